@@ -15,13 +15,13 @@
 // the handoff crosses PCIe.  One CTA of five warps (three for rows of at most 512
 // bytes) per query, persistent: CTA i owns slot i of the visited-set pool
 // (visited.cu), starts on query i and claims further queries from a counter.
-// Warp 0 is the heap warp (it runs upstream's heap routines), the other warps
-// gather: adjacency row, visited marks, vector rows, distances.  Three serial
-// pieces of upstream's routine -- pushing the seeds into the open heap of the
-// two-expansion stage, seeding the full-graph stage, merging seeds and result --
-// are computed from their outcome when the keys involved are pairwise different
-// (brief_search, the seeding in search_stage, select_sort_output) and run as
-// upstream wrote them otherwise.  In the full-graph stage the two sides overlap: the node the next
+// Warp 0 is the heap warp, the other warps gather: adjacency row, visited marks,
+// vector rows, distances.  Four serial pieces of upstream's routine -- the result
+// heap, pushing the seeds into the open heap of the two-expansion stage, seeding the
+// full-graph stage, merging seeds and result -- are computed from their outcome when
+// the keys involved are pairwise different (TopList, brief_search, the seeding in
+// heap_loop, select_sort_output and merge_sorted_output) and run as upstream wrote
+// them otherwise.  In the full-graph stage the two sides overlap: the node the next
 // pop will return is known as soon as the distances of the current expansion are
 // (it is the better of the open heap's root and the best new neighbour -- a new
 // key below the root always sifts up to the root, equal keys never pass it), so
@@ -32,13 +32,14 @@
 // are never looked at again.  The sub-graph stage does not speculate: its marks
 // are inherited by the full-graph stage.  Semantics are upstream's, operation
 // for operation:
-//   * the result heap (H entries) and the open heap (2H entries) are upstream's
-//     array heaps with upstream's routines (extension/inc/heapq.cuh:13-87) --
-//     heap_replace evicts the leaf reached by walking larger children, not the
-//     maximum, so the layout is part of the result; they live in shared memory,
-//     stored 1-based as {key, id} pairs so that both children of a node come in
-//     one 16-byte load, and are driven by the 32 lanes of the heap warp together
-//     (see the routines below);
+//   * the open heap (2H entries) is upstream's array heap with upstream's routines
+//     (extension/inc/heapq.cuh:13-87) -- heap_replace evicts the leaf reached by
+//     walking larger children, not the maximum, so the layout is part of the
+//     result; it lives in shared memory, stored 1-based as {key, id} pairs so that
+//     both children of a node come in one 16-byte load, and is driven by the 32
+//     lanes of the heap warp together (see the routines below).  So does the result
+//     heap (H entries) where H > 256; up to there the results are a sorted list in
+//     registers (TopList);
 //   * H follows upstream's CPU dispatch (traverse_cpu.cpp:228-254);
 //   * exact visited marks (extension/inc/bitmask.hpp:12-45) shared by the two
 //     stages of a query, as upstream shares one marker between them;
@@ -252,6 +253,211 @@ __device__ __forceinline__ void warp_replace(HeapEntry *h, int n, float k, int32
     __syncwarp();
 }
 
+// The same operations with the outcome of every comparison kept: bit n of a set of
+// words (uniform over the warp, in registers) says whether the right child of node n
+// is strictly larger (open heap) or smaller (result heap).  The walk is then a few
+// integer instructions instead of two rounds of loads and ballots; lane t looks at the
+// path node at depth t + 1, its parent and its sibling, and says whether the bit of
+// the parent (depth t) turns.  Heaps of up to 64 W nodes.
+template <int W> struct PathBits {
+    static constexpr int kUniform = W > 4 ? 2 : W;  // words every lane holds
+    uint32_t w[kUniform];
+    uint32_t deep;  // W = 8: lane i holds word i (six registers less, two shuffles more)
+
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int i = 0; i < kUniform; ++i) w[i] = 0;
+        deep = 0;
+    }
+    __device__ __forceinline__ void build_larger(const HeapEntry *h, int n, int lane) {
+        deep = 0;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+            const int node = 32 * i + lane;
+            bool right = false;
+            if (node >= 1 && 2 * node + 1 <= n) {
+                const int4 p = *reinterpret_cast<const int4 *>(h + 2 * node);
+                right = __int_as_float(p.z) > __int_as_float(p.x);
+            }
+            const uint32_t word = __ballot_sync(kAll, right);
+            if (i < kUniform) w[i < kUniform ? i : 0] = word;
+            else if (lane == i) deep = word;
+        }
+    }
+    // The leaf at the end of the path in a heap of n nodes.  All nodes of the first kSure
+    // levels below the root exist for every n that comes with this many words.
+    __device__ __forceinline__ int leaf(int n) const {
+        constexpr int kDepth = W == 1 ? 6 : W == 2 ? 7 : W == 4 ? 8 : 9;
+        constexpr int kSure = W == 1 ? 3 : W == 2 ? 4 : W == 4 ? 6 : 7;
+        unsigned a = 1;
+#pragma unroll
+        for (int l = 0; l < kDepth; ++l) {
+            uint32_t word = 0;
+            if (l < 5) word = w[0];
+            if (l == 5 && W >= 2) word = w[W >= 2 ? 1 : 0];
+            if (l == 6 && W == 4) word = (a & 32u) ? w[W == 4 ? 3 : 0] : w[W == 4 ? 2 : 0];
+            if ((l == 6 || l == 7) && W == 8) word = __shfl_sync(kAll, deep, a >> 5);
+            const unsigned c = (a << 1) | (__funnelshift_r(word, 0u, a) & 1u);
+            a = l < kSure || 2 * a <= static_cast<unsigned>(n) ? c : a;
+        }
+        return static_cast<int>(a);
+    }
+    // Turns the bits of the path's nodes for which the lane of their depth says so.
+    __device__ __forceinline__ void turn(bool flip, int leaf, int depth, int lane) {
+        const unsigned F = __ballot_sync(kAll, flip);
+        w[0] ^= __reduce_or_sync(kAll, flip && lane < 5 ? 1u << ((leaf >> (depth - lane)) & 31) : 0u);
+        auto node = [&](int t) { return leaf >> ((depth - t) & 31); };  // of the path, at depth t
+        auto bit = [&](int t) { return ((F >> t) & 1u) << (node(t) & 31); };
+        if constexpr (W >= 2) w[1] ^= bit(5);
+        if constexpr (W == 4) {
+            w[2] ^= (node(6) & 32) ? 0u : bit(6);
+            w[3] ^= (node(6) & 32) ? bit(6) : 0u;
+        }
+        if constexpr (W == 8) {
+            deep ^= lane == node(6) >> 5 ? bit(6) : 0u;
+            deep ^= lane == node(7) >> 5 ? bit(7) : 0u;
+        }
+    }
+};
+
+// What lane t sees of a path: the node at depth t + 1 and its sibling's key.
+struct PathLane {
+    int depth, node;
+    bool on, sib;  // the path reaches this lane; the node has a sibling
+    float sk;
+};
+__device__ __forceinline__ PathLane path_lane(const HeapEntry *h, int n, int leaf, int lane) {
+    PathLane p;
+    p.depth = 31 - __clz(leaf);
+    p.on = lane < p.depth;
+    p.node = p.on ? leaf >> (p.depth - 1 - lane) : 2;
+    p.sib = p.on && (p.node | 1) <= n;
+    p.sk = h[p.sib ? p.node ^ 1 : p.node].k;
+    return p;
+}
+
+// warp_sink over the bits of the smaller children (result heap).
+template <int W>
+__device__ __forceinline__ void bit_sink(HeapEntry *h, int n, HeapEntry me, PathBits<W> &smaller,
+                                         int lane) {
+    const int leaf = smaller.leaf(n);
+    const PathLane p = path_lane(h, n, leaf, lane);
+    const HeapEntry e = h[p.node];
+    const unsigned m = __ballot_sync(kAll, p.on && e.k < me.k);
+    const int cnt = __ffs(~m) - 1;
+    const float below = __shfl_down_sync(kAll, e.k, 1);
+    const float nk = lane + 1 == cnt ? me.k : below;  // the node's new key (lane < cnt)
+    __syncwarp();
+    if (lane < cnt) h[p.node >> 1] = e;
+    if (lane == 0) h[cnt == 0 ? 1 : leaf >> (p.depth - cnt)] = me;
+    // the path went to the node: right if strictly smaller than its sibling
+    const bool stays = (p.node & 1) ? nk < p.sk : !(p.sk < nk);
+    smaller.turn(lane < cnt && p.sib && !stays, leaf, p.depth, lane);
+    __syncwarp();
+}
+
+// warp_pop of a heap with the bits of its larger children (open heap).
+template <int W>
+__device__ __forceinline__ HeapEntry bit_pop(HeapEntry *h, int n, PathBits<W> &larger, int lane,
+                                             const WalkLane &L) {
+    const HeapEntry out = h[1];
+    const int leaf = warp_walk<false>(h, n, lane, L);
+    const PathLane p = path_lane(h, n, leaf, lane);
+    const HeapEntry e = h[p.node];
+    const unsigned m = __ballot_sync(kAll, p.on && e.k < CUDART_INF_F);
+    const int cnt = __ffs(~m) - 1;
+    const float below = __shfl_down_sync(kAll, e.k, 1);
+    const float nk = lane + 1 == cnt ? CUDART_INF_F : below;
+    __syncwarp();
+    if (lane < cnt) h[p.node >> 1] = e;
+    if (lane == 0) h[cnt == 0 ? 1 : leaf >> (p.depth - cnt)] = HeapEntry{CUDART_INF_F, -1};
+    const bool was = (p.node & 1) ? e.k > p.sk : p.sk > e.k;
+    const bool is = (p.node & 1) ? nk > p.sk : p.sk > nk;
+    larger.turn(lane < cnt && p.sib && was != is, leaf, p.depth, lane);
+    __syncwarp();
+    return out;
+}
+
+// warp_replace over the bits of the larger children (open heap).
+template <int W>
+__device__ __forceinline__ void bit_replace(HeapEntry *h, int n, float k, int32_t v,
+                                            PathBits<W> &larger, int lane) {
+    const int leaf = larger.leaf(n);
+    const PathLane p = path_lane(h, n, leaf, lane);
+    const HeapEntry e = h[p.node >> 1];
+    if (k >= h[leaf].k) return;
+    const unsigned m = __ballot_sync(kAll, p.on && e.k > k);
+    const int s = m != 0 ? __ffs(m) - 1 : p.depth;  // depth at which the new entry lands
+    const bool moves = p.on && lane >= s;
+    __syncwarp();
+    if (moves) h[p.node] = e;
+    if (lane == 0) h[leaf >> (p.depth - s)] = HeapEntry{k, v};
+    const float nk = moves ? e.k : k;  // the node's new key (lane >= s - 1)
+    const bool stays = (p.node & 1) ? nk > p.sk : !(p.sk > nk);
+    larger.turn(p.sib && lane + 1 >= s && !stays, leaf, p.depth, lane);
+    __syncwarp();
+}
+
+// ---- the H best results, in the registers of the heap warp -----------------------
+// Upstream keeps them in an array heap (heap_pushpop, heapq.cuh:79-87).  With pairwise
+// different distances its layout is never seen: a push drops the worst entry, the root
+// is the largest distance, and the pops of the end come out sorted.  So up to 256 of
+// them are held sorted, ascending, in registers (position i of the list in slot
+// i + 32 R - H, slot s in register s / 32 of lane s mod 32; the slots before hold -inf
+// and never move): an insertion is one rotation by a lane per register, about 70 cycles
+// where heap_pushpop took 600 to 900.  Where distances are equal the layout decides
+// which of two entries is dropped or comes first; the admitted entries are logged in
+// shared memory, and a merge that meets equal distances among the entries that matter
+// replays the log through heap_pushpop (search_stage).
+//
+// What it gave, with the open heap's comparison bits (PathBits) and the merge of two
+// sorted lists: the launch in ms, heaps as arrays -> now: 1024 queries of 768 dimensions
+// at ef 128 2.29 -> 2.11, 8192 of them 16.1 -> 15.4; 96 dimensions at ef 256: 1024 2.81 ->
+// 1.99, 16384 13.5 -> 12.3; 200 dimensions at ef 192, k 100: 1024 2.29 -> 1.97; seven
+// queries of 96 dimensions at ef 96 0.40 -> 0.31.
+template <int R> struct TopList {
+    float k[R];
+    int32_t v[R];
+
+    __device__ __forceinline__ void clear(int H, int lane) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            k[r] = 32 * r + lane < 32 * R - H ? -CUDART_INF_F : CUDART_INF_F;
+            v[r] = -1;
+        }
+    }
+    __device__ __forceinline__ float worst() const { return __shfl_sync(kAll, k[R - 1], 31); }
+    // The last entry leaves; true if the one before it is its equal.
+    __device__ __forceinline__ bool worst_twice(float worst_k) const {
+        return __shfl_sync(kAll, k[R - 1], 30) == worst_k;
+    }
+    __device__ __forceinline__ void insert(float nk, int32_t nv, int lane) {
+        // downwards, so that few rotated copies are alive at a time
+        const int from = (lane + 31) & 31;
+        float pk = __shfl_sync(kAll, k[R - 1], from);
+        int32_t pv = __shfl_sync(kAll, v[R - 1], from);
+#pragma unroll
+        for (int r = R - 1; r >= 0; --r) {
+            const float below_k = r > 0 ? __shfl_sync(kAll, k[r > 0 ? r - 1 : 0], from) : -CUDART_INF_F;
+            const int32_t below_v = r > 0 ? __shfl_sync(kAll, v[r > 0 ? r - 1 : 0], from) : -1;
+            // the entry one position before this one
+            const float qk = lane != 0 ? pk : below_k;
+            const int32_t qv = lane != 0 ? pv : below_v;
+            if (k[r] > nk) {
+                v[r] = qk > nk ? qv : nv;
+                k[r] = qk > nk ? qk : nk;
+            }
+            pk = below_k;
+            pv = below_v;
+        }
+    }
+};
+
+// Registers per lane of the list for a capacity of H; 0: the array heap is used.
+__host__ __device__ constexpr int list_regs_for(int H) {
+    return H <= 64 ? 2 : H <= 128 ? 4 : H <= 256 ? 8 : 0;
+}
+
 // ---- distances: one warp per row, two rows in flight ----------------------------
 __device__ __forceinline__ float ref_stripe(float acc, float4 c, float4 p) {
     const float dx = __fsub_rn(c.x, p.x), dy = __fsub_rn(c.y, p.y);
@@ -340,7 +546,8 @@ __device__ __forceinline__ float staged_row(const float *stage, const float *q_s
 struct RefShared {
     float *q;          // [d]
     HeapEntry *open;   // [2H + 2]
-    HeapEntry *buf;    // [H + 2]
+    HeapEntry *buf;    // [H + 2] result heap; with the result list in registers: the first
+                       //         H entries of the log, the list once the stage is over
     int32_t *c_id;     // [n_cand] seeds of the running stage, then its output
     float *c_d;
     int32_t *nb_id;    // [2][kMaxDegree] unvisited neighbours of an expanded node
@@ -357,12 +564,22 @@ struct RefCtl {
     int root_v[2];
     int guess[2];       // node the gather warps prepared expansion i for
     int n_new[2];       // unvisited neighbours found for expansion i
-    int tie;            // select_sort_output gave up: run upstream's sequence
+    int tie;            // the merge gave up: run upstream's sequence
     unsigned next;      // the query claimed for the CTA's next round
-    int sorted;         // the last select_sort_output wrote its output (strictly ascending)
+    int sorted;         // the stage's output: kAscending | kHeadStrict
     int n_taken, n_equal;
     int marker;
+    float amb;          // TopList: smallest distance of which one of several was dropped
+    int n_log;          //          entries admitted
+    int st[4];          // expansions and evaluations of the two stages
+    int rerun;          //          the query has to be run on the array heaps
 };
+constexpr int kAscending = 1;   // the real entries ascend
+constexpr int kHeadStrict = 2;  // the first kSeedHead of them strictly
+constexpr int kSeedHead = 26;   // entries the seeding of the open heap may look at
+
+// Every thread of the CTA, whichever side of the warp specialisation it is on.
+__device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 0;" ::: "memory"); }
 
 __device__ __forceinline__ void gather_sync() {  // the gather warps only
     asm volatile("bar.sync 1, %0;" ::"r"(static_cast<int>(blockDim.x) - 32) : "memory");
@@ -452,20 +669,35 @@ __device__ __forceinline__ void gather_node(const RefineArgs &A, const RefShared
 // smallest distances; one equal to the current worst stays out), pops the H - k_out
 // worst entries and stores the others worst first, i.e. ascending.  When the
 // distances that matter are pairwise different, that is the n_real smallest of
-// (result heap + seeds) in ascending order, whatever the heaps looked like on the
+// (results + seeds) in ascending order, whatever the heaps looked like on the
 // way.  So: (1) a radix select over the float bit patterns (non-negative floats
 // order like their bits; eight 4-bit passes with 16 shared counters) finds the H-th
 // smallest distance T, (2) the entries below T and as many of those equal to T as
 // still fit are gathered into the open heap's memory (dead by now), (3) a bitonic
-// network sorts them, (4) the first n_real are stored.  More entries equal to T than
-// fit, two equal distances among the chosen (pads of the result heap, (-1, +inf),
-// excepted: they are interchangeable), or a distance that is negative or NaN make
-// the outcome depend on upstream's exact sequence: nothing is written then and the
-// caller runs that sequence.  Returns true (CTA-uniform) if the output is written.
-__device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, int n_seed,
-                                                   int n_real, int k_out, RefCtl *ctl) {
+// network sorts them, (4) the first n_real are stored.
+// Which equal distances matter: those among the first n_check entries and the one
+// behind them (pads, (-1, +inf), excepted: they are interchangeable).  The sub-graph
+// stage of a search that goes on hands n_check = max(k, kSeedHead): entries further
+// back are too far for the seeding of the full-graph stage, and the final k are no
+// larger than the k smallest here -- exchanging two ids of equal distance behind
+// them exchanges these ids in every later heap and nothing else.  Equal distances
+// that matter, or a distance that is negative or NaN, make the outcome depend on
+// upstream's exact sequence: nothing is written then and the caller runs that
+// sequence.  Returns true (CTA-uniform) if the output is written.
+template <int R>
+__device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, int seed_lo,
+                                                   int n_seed, int n_real, int k_out, int n_check,
+                                                   RefCtl *ctl) {
     const int tid = threadIdx.x, n_thr = blockDim.x;
-    const int N = H + n_seed;
+    const int32_t *c_id = S.c_id + seed_lo;
+    const float *c_d = S.c_d + seed_lo;
+    // the array heap holds negated distances, the dumped list distances
+    auto result_at = [&](int x) {
+        HeapEntry e = S.buf[1 + x];
+        if (R == 0) e.k = -e.k;
+        return e;
+    };
+    const int N = H + n_seed - seed_lo;
     int *bins = reinterpret_cast<int *>(S.open);  // 16 counters, then the gathered entries
     HeapEntry *a = S.open;
     if (tid == 0) {
@@ -484,10 +716,10 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
         for (int x = tid; x < N; x += n_thr) {
             float dx;
             if (x < H) {
-                dx = -S.buf[1 + x].k;
+                dx = result_at(x).k;
             } else {
-                if (S.c_id[x - H] < 0) continue;
-                dx = S.c_d[x - H];
+                if (c_id[x - H] < 0) continue;
+                dx = c_d[x - H];
             }
             if (!(dx >= 0.0f)) bad = true;
             const unsigned key = __float_as_uint(dx);
@@ -514,7 +746,7 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
         mask |= 15u << shift;
     }
     const unsigned T = prefix;  // `want` of the at_T entries equal to T are needed
-    if (at_T > want && T != __float_as_uint(CUDART_INF_F)) bad = true;
+    if (n_check >= H && at_T > want && T != __float_as_uint(CUDART_INF_F)) bad = true;
     if (bad) ctl->tie = 1;
     __syncthreads();
     if (ctl->tie != 0) return false;
@@ -525,12 +757,11 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
     for (int x = tid; x < N; x += n_thr) {
         HeapEntry e;
         if (x < H) {
-            e = S.buf[1 + x];
-            e.k = -e.k;
+            e = result_at(x);
         } else {
-            e.v = S.c_id[x - H];
+            e.v = c_id[x - H];
             if (e.v < 0) continue;
-            e.k = S.c_d[x - H];
+            e.k = c_d[x - H];
         }
         const unsigned key = __float_as_uint(e.k);
         bool take = key < T;
@@ -554,8 +785,8 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
             __syncthreads();
         }
     }
-    bool tie = false;
-    for (int i = tid; i + 1 < H; i += n_thr)
+    bool tie = R > 0 && ctl->amb < CUDART_INF_F && ctl->amb <= a[n_check - 1].k;
+    for (int i = tid; i < n_check && i + 1 < H; i += n_thr)
         if (a[i].k == a[i + 1].k && (a[i].v >= 0 || a[i + 1].v >= 0)) tie = true;
     if (tie) ctl->tie = 1;
     __syncthreads();
@@ -569,6 +800,167 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
     return true;
 }
 
+// The same end when the seeds ascend (full-graph stage): results and seeds are two
+// sorted lists, an entry's place in the union is its own index plus the entries of
+// the other list before it (a binary search).  Writes the first n_real.
+__device__ __forceinline__ bool merge_sorted_output(const RefShared &S, const HeapEntry *list,
+                                                    int H, int seed_lo, int n_seed, int n_real,
+                                                    int k_out, RefCtl *ctl) {
+    const int tid = threadIdx.x, n_thr = blockDim.x;
+    const int ny = n_seed - seed_lo;
+    HeapEntry *a = S.open;  // [n_real + 1], in front of `list`: the last one only to compare with
+    if (tid == 0) {
+        ctl->tie = 0;
+        a[n_real] = HeapEntry{CUDART_INF_F, -1};  // should the union end before it
+    }
+    __syncthreads();
+    for (int x = tid; x < H + ny; x += n_thr) {
+        const bool res = x < H;
+        const int own = res ? x : x - H;
+        const HeapEntry e = res ? list[own] : HeapEntry{S.c_d[seed_lo + own], S.c_id[seed_lo + own]};
+        if (own > n_real) continue;
+        int lo = 0, hi = res ? ny : H;  // entries of the other list in front of e
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            const float o = res ? S.c_d[seed_lo + mid] : list[mid].k;
+            if (res ? o < e.k : o <= e.k) lo = mid + 1; else hi = mid;
+        }
+        if (own + lo <= n_real) a[own + lo] = e;
+    }
+    __syncthreads();
+    bool tie = ctl->amb < CUDART_INF_F && ctl->amb <= a[n_real - 1].k;
+    for (int i = tid; i < n_real; i += n_thr)
+        if (a[i].k == a[i + 1].k && (a[i].v >= 0 || a[i + 1].v >= 0)) tie = true;
+    if (tie) ctl->tie = 1;
+    __syncthreads();
+    if (ctl->tie != 0) return false;
+    for (int r = tid; r < n_real; r += n_thr) {
+        S.c_id[k_out - n_real + r] = a[r].v;
+        S.c_d[k_out - n_real + r] = a[r].k;
+    }
+    return true;
+}
+
+__device__ __forceinline__ RefShared ref_shared(const RefineArgs &A, unsigned char *smem) {
+    RefShared S;
+    S.q = reinterpret_cast<float *>(smem);
+    S.open = reinterpret_cast<HeapEntry *>(S.q + A.d);
+    S.buf = S.open + 2 * A.H + 2;
+    S.c_id = reinterpret_cast<int32_t *>(S.buf + A.H + 2);
+    S.c_d = reinterpret_cast<float *>(S.c_id + A.n_cand);
+    S.nb_id = reinterpret_cast<int32_t *>(S.c_d + A.n_cand);
+    S.nb_d = reinterpret_cast<float *>(S.nb_id + 2 * kMaxDegree);
+    S.stage = S.nb_d + 2 * kMaxDegree;
+    return S;
+}
+
+extern __shared__ __align__(16) unsigned char ref_smem[];
+
+// The heap warp's side of a stage: the result list (or the array heap, R = 0), the
+// log, the counters.
+template <int R> struct HeapSide {
+    TopList<R> top;
+    float worst;
+    int n_log;
+    PathBits<R> larger;  // of the open heap
+
+    __device__ __forceinline__ void clear(int H, int lane) {
+        top.clear(H, lane);
+        worst = CUDART_INF_F;
+        n_log = 0;
+    }
+    // the open heap, once it holds its seeds
+    __device__ __forceinline__ void open_filled(const RefShared &S, int n, int lane) {
+        larger.build_larger(S.open, n, lane);
+    }
+    __device__ __forceinline__ void open_push(const RefShared &S, int n, float k, int32_t v,
+                                              int lane, const WalkLane &) {
+        bit_replace(S.open, n, k, v, larger, lane);
+    }
+    __device__ __forceinline__ HeapEntry open_pop(const RefShared &S, int n, int lane,
+                                                  const WalkLane &WL) {
+        return bit_pop(S.open, n, larger, lane, WL);
+    }
+    __device__ __forceinline__ float worst_of(const RefShared &) const { return worst; }
+    // heap_update (:23-39) over the n_new neighbours in buffer nb: every distance below
+    // the worst result is admitted, in row order; f(distance, id, index) follows.
+    template <class F>
+    __device__ __forceinline__ void admit(const RefShared &S, const int32_t *nb_id,
+                                          const float *nb_d, int n_new, int log_room, int H,
+                                          int lane, const WalkLane &, RefCtl *ctl, F f) {
+        for (int c = 0; c < n_new; c += 32) {
+            const bool in = c + lane < n_new;
+            const float dist = in ? nb_d[c + lane] : CUDART_INF_F;
+            const int32_t id = in ? nb_id[c + lane] : -1;
+            if (!(dist >= 0.0f)) ctl->rerun = 1;  // NaN: see search_stage
+            unsigned ahead = kAll;
+            for (;;) {
+                const unsigned m = __ballot_sync(kAll, dist < worst) & ahead;
+                if (m == 0) break;
+                const int j = __ffs(m) - 1;
+                ahead = 0xfffffffeu << j;
+                const float nk = __shfl_sync(kAll, dist, j);
+                const int32_t nv = __shfl_sync(kAll, id, j);
+                if (top.worst_twice(worst)) ctl->amb = fminf(ctl->amb, worst);  // all lanes alike
+                top.insert(nk, nv, lane);
+                worst = top.worst();
+                if (lane == 0) {
+                    if (n_log < min(H, log_room)) {
+                        S.buf[1 + n_log] = HeapEntry{nk, nv};
+                    } else if (n_log < log_room) {
+                        S.c_id[n_log - H] = nv;
+                        S.c_d[n_log - H] = nk;
+                    }
+                }
+                ++n_log;
+                f(nk, nv, c + j);
+            }
+        }
+    }
+    // after the last expansion: the list to shared memory, ascending
+    __device__ __forceinline__ void finish(HeapEntry *list, int H, int lane, RefCtl *ctl) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = 32 * r + lane - (32 * R - H);
+            if (i >= 0) list[i] = HeapEntry{top.k[r], top.v[r]};
+        }
+        ctl->n_log = n_log;
+    }
+};
+
+template <> struct HeapSide<0> {
+    __device__ __forceinline__ void clear(int, int) {}
+    __device__ __forceinline__ void open_filled(const RefShared &, int, int) {}
+    __device__ __forceinline__ void open_push(const RefShared &S, int n, float k, int32_t v,
+                                              int lane, const WalkLane &WL) {
+        warp_replace(S.open, n, k, v, lane, WL);
+    }
+    __device__ __forceinline__ HeapEntry open_pop(const RefShared &S, int n, int lane,
+                                                  const WalkLane &WL) {
+        return warp_pop(S.open, n, lane, WL);
+    }
+    __device__ __forceinline__ float worst_of(const RefShared &S) const { return -S.buf[1].k; }
+    template <class F>
+    __device__ __forceinline__ void admit(const RefShared &S, const int32_t *nb_id,
+                                          const float *nb_d, int n_new, int, int H, int lane,
+                                          const WalkLane &WL, RefCtl *, F f) {
+        for (int j = 0; j < n_new; ++j) {
+            const float dist = nb_d[j];
+            if (dist >= -S.buf[1].k) continue;
+            warp_pushpop(S.buf, H, -dist, nb_id[j], lane, WL);
+            f(dist, nb_id[j], j);
+        }
+    }
+    __device__ __forceinline__ void finish(HeapEntry *, int, int, RefCtl *) {}
+};
+
+__device__ __forceinline__ void count_expansion(int *st, int n_new, int lane) {
+    if (lane == 0) {
+        ++st[0];
+        st[1] += n_new;
+    }
+}
+
 // A search of exactly two expansions (the sub-graph stage: REFINE_STEP = 2,
 // traverse_cpu.cpp:317-326) without the open heap.  heap_replace only ever drops or
 // evicts an entry that is no smaller than the leaf at the end of a larger-child
@@ -577,20 +969,16 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
 // walk) -- so the two smallest keys ever offered are in the heap when they are
 // popped, and with pairwise different keys the two pops are simply: the smallest
 // seed, then the smaller of the second-smallest seed and the best neighbour
-// admitted during the first expansion.  The result heap is kept exactly as
-// upstream keeps it (its worst entry decides admissions and the stop test).
+// admitted during the first expansion.  The results are kept exactly as
+// upstream keeps them (the worst decides admissions and the stop test).
 // Whenever the keys that matter are not pairwise different the layout of the open
 // heap decides: with equal smallest seeds nothing is done and false is returned (the
 // caller runs upstream's sequence); a tie met at the second pop is settled by
 // building the open heap after all, in upstream's order, and popping it.
-// Called by all threads after the seeds are marked; returns CTA-uniformly.
-__device__ __forceinline__ bool brief_search(const RefineArgs &A, const RefShared &S,
-                                             const RefGraph &G, uint8_t *vis, uint8_t marker,
-                                             int n_seed, RefCtl *ctl, const WalkLane &WL,
-                                             int &n_expand, int &n_eval, int *prof,
-                                             long long &prof_t) {
-    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n_thr = blockDim.x;
-    const int H = A.H;
+// Called by all threads after the seeds are marked; returns CTA-uniformly whether
+// ctl->m1 .. c2 hold what brief_search needs.
+__device__ __forceinline__ bool brief_prepare(const RefShared &S, int n_seed, RefCtl *ctl) {
+    const int tid = threadIdx.x, n_thr = blockDim.x;
     constexpr unsigned long long kNone = ~0ull;
     if (tid == 0) {
         ctl->m1 = ctl->m2 = kNone;
@@ -624,97 +1012,299 @@ __device__ __forceinline__ bool brief_search(const RefineArgs &A, const RefShare
         if (__float_as_uint(S.c_d[i]) == static_cast<unsigned>(m2 >> 32)) atomicAdd(&ctl->c2, 1);
     }
     __syncthreads();
-    if (m1 == kNone) return true;  // no seed at all: the first pop ends the search
-    // first pop: the smallest seed; the result heap is empty, the stop test passes
-    const int u1 = S.c_id[i1];
-    if (w > 0) gather_node(A, S, G, vis, marker, ctl, u1, 0, w - 1, lane, prof, prof_t);
-    __syncthreads();
-    if (w == 0) {
-        const int n_new = ctl->n_new[0];
-        ++n_expand;
-        n_eval += n_new;
-        unsigned long long admitted = 0;
-        float best = CUDART_INF_F;
-        int best_j = -1;
-        bool best_twice = false;
-        for (int j = 0; j < n_new; ++j) {  // heap_update (:23-39) without the open heap
-            const float dist = S.nb_d[j];
-            if (dist >= -S.buf[1].k) continue;
-            warp_pushpop(S.buf, H, -dist, S.nb_id[j], lane, WL);
-            admitted |= 1ull << j;
-            if (dist < best) {
-                best = dist;
-                best_j = j;
-                best_twice = false;
-            } else if (dist == best) {
-                best_twice = true;
-            }
-        }
-        // second pop
-        const bool seed_left = m2 != kNone;
-        const float seed_k = seed_left ? S.c_d[i2] : CUDART_INF_F;
-        int u2 = -1;
-        float k2 = CUDART_INF_F;
-        bool unsure = false;
-        if (best_j >= 0 && (!seed_left || best < seed_k)) {
-            u2 = S.nb_id[best_j];
-            k2 = best;
-            unsure = best_twice;
-        } else if (seed_left && (best_j < 0 || seed_k < best)) {
-            u2 = S.c_id[i2];
-            k2 = seed_k;
-            unsure = ctl->c2 != 0;
-        } else if (seed_left) {  // equal
-            unsure = true;
-        }
-        if (unsure) {  // upstream's sequence on the open heap
-            for (int i = 0; i < n_seed; ++i) {
-                const int id = S.c_id[i];
-                if (id >= 0) warp_replace(S.open, 2 * H, S.c_d[i], id, lane, WL);
-            }
-            warp_pop(S.open, 2 * H, lane, WL);
-            for (int j = 0; j < n_new; ++j)
-                if ((admitted >> j) & 1ull) warp_replace(S.open, 2 * H, S.nb_d[j], S.nb_id[j], lane, WL);
-            const HeapEntry nx = warp_pop(S.open, 2 * H, lane, WL);
-            u2 = nx.v;
-            k2 = nx.k;
-        }
-        if (u2 >= 0 && k2 >= -S.buf[1].k) u2 = -1;  // :86-90
-        if (lane == 0) ctl->pop_u[1] = u2;
-    }
-    __syncthreads();
-    const int u2 = ctl->pop_u[1];
-    if (u2 < 0) return true;
-    if (w > 0) gather_node(A, S, G, vis, marker, ctl, u2, 1, w - 1, lane, prof, prof_t);
-    __syncthreads();
-    if (w == 0) {
-        const int n_new = ctl->n_new[1];
-        const int32_t *nb_id = S.nb_id + kMaxDegree;
-        const float *nb_d = S.nb_d + kMaxDegree;
-        ++n_expand;
-        n_eval += n_new;
-        for (int j = 0; j < n_new; ++j) {
-            const float dist = nb_d[j];
-            if (dist >= -S.buf[1].k) continue;
-            warp_pushpop(S.buf, H, -dist, nb_id[j], lane, WL);
-        }
-    }
     return true;
+}
+
+// The heap warp's half; the gather warps run the two expansions (search_stage).
+template <int R>
+__device__ __forceinline__ void brief_search(const RefineArgs &A, const RefShared &S, int n_seed,
+                                             RefCtl *ctl, HeapSide<R> &side, const WalkLane &WL,
+                                             int lane, int *st) {
+    constexpr unsigned long long kNone = ~0ull;
+    const int H = A.H;
+    const unsigned long long m1 = ctl->m1, m2 = ctl->m2;
+    if (m1 == kNone) return;  // no seed at all: the first pop ends the search
+    const int i2 = static_cast<int>(m2 & 0xffffffffu);
+    // first pop: the smallest seed; there is no result yet, the stop test passes
+    cta_sync();  // its neighbours are in buffer 0
+    const int n_new = ctl->n_new[0];
+    count_expansion(st, n_new, lane);
+    unsigned long long admitted = 0;
+    float best = CUDART_INF_F;
+    int best_j = -1;
+    bool best_twice = false;
+    side.admit(S, S.nb_id, S.nb_d, n_new, 0, H, lane, WL, ctl,
+               [&](float dist, int32_t, int j) {  // heap_update without the open heap
+                   admitted |= 1ull << j;
+                   if (dist < best) {
+                       best = dist;
+                       best_j = j;
+                       best_twice = false;
+                   } else if (dist == best) {
+                       best_twice = true;
+                   }
+               });
+    // second pop
+    const bool seed_left = m2 != kNone;
+    const float seed_k = seed_left ? S.c_d[i2] : CUDART_INF_F;
+    int u2 = -1;
+    float k2 = CUDART_INF_F;
+    bool unsure = false;
+    if (best_j >= 0 && (!seed_left || best < seed_k)) {
+        u2 = S.nb_id[best_j];
+        k2 = best;
+        unsure = best_twice;
+    } else if (seed_left && (best_j < 0 || seed_k < best)) {
+        u2 = S.c_id[i2];
+        k2 = seed_k;
+        unsure = ctl->c2 != 0;
+    } else if (seed_left) {  // equal
+        unsure = true;
+    }
+    if (unsure) {  // upstream's sequence on the open heap
+        for (int i = 0; i < n_seed; ++i) {
+            const int id = S.c_id[i];
+            if (id >= 0) warp_replace(S.open, 2 * H, S.c_d[i], id, lane, WL);
+        }
+        warp_pop(S.open, 2 * H, lane, WL);
+        for (int j = 0; j < n_new; ++j)
+            if ((admitted >> j) & 1ull) warp_replace(S.open, 2 * H, S.nb_d[j], S.nb_id[j], lane, WL);
+        const HeapEntry nx = warp_pop(S.open, 2 * H, lane, WL);
+        u2 = nx.v;
+        k2 = nx.k;
+    }
+    if (u2 >= 0 && k2 >= side.worst_of(S)) u2 = -1;  // :86-90
+    if (lane == 0) ctl->pop_u[1] = u2;
+    cta_sync();
+    if (u2 < 0) return;
+    cta_sync();  // the second expansion is in buffer 1
+    count_expansion(st, ctl->n_new[1], lane);
+    side.admit(S, S.nb_id + kMaxDegree, S.nb_d + kMaxDegree, ctl->n_new[1], 0, H, lane, WL, ctl,
+               [](float, int32_t, int) {});
+}
+
+// The heap warp's half of the general search (:64-136).
+template <int R>
+__device__ __forceinline__ void heap_loop(const RefineArgs &A, const RefShared &S, int n_seed,
+                                          int seed_lo, int max_iter, bool closed_form, int log_room,
+                                          RefCtl *ctl, HeapSide<R> &side, const WalkLane &WL,
+                                          int lane, int *st, int *prof, long long &prof_t) {
+    (void)prof; (void)prof_t;
+    const int H = A.H;
+    if (closed_form) {
+        // The real seeds are c[seed_lo ..] in ascending order, the first kSeedHead of them
+        // strictly.  Every key offered to heap_replace is then no smaller than all keys in
+        // the heap: it replaces a +inf leaf and climbs to just below a real entry, or meets
+        // a real leaf and is dropped -- which of the two depends on the count of
+        // seeds before it only.  Seed 0 ends at heap index 0, seeds 2t - 1 and 2t
+        // at the two rightmost nodes of level t (2^(t+1) - 3 and 2^(t+1) - 2,
+        // 0-based) while those exist; all later seeds are dropped.  Checked
+        // against heap_replace for every heap size and seed count on the host.
+        const int t = (lane + 1) >> 1;
+        const int pos = lane == 0 ? 0 : (1 << (t + 1)) - 3 + ((lane & 1) ? 0 : 1);
+        const int at = seed_lo + lane;
+        // (heap_replace drops an infinite key)
+        if (lane < 25 && pos < 2 * H && at < n_seed && S.c_id[at] >= 0 && S.c_d[at] < CUDART_INF_F)
+            S.open[1 + pos] = HeapEntry{S.c_d[at], S.c_id[at]};
+        __syncwarp();
+    } else {
+        for (int i = 0; i < n_seed; ++i) {
+            const int id = S.c_id[i];
+            if (id >= 0) warp_replace(S.open, 2 * H, S.c_d[i], id, lane, WL);
+        }
+    }
+    side.open_filled(S, 2 * H, lane);
+    PA_TICK(1);
+    // :82-136.  Expansion i uses slot i & 1 of the control block and of the
+    // neighbour buffers.  Per expansion one CTA-wide barrier: behind it the heap
+    // warp has popped node i (or ended the search) and -- when speculating --
+    // the gather warps have prepared the node they expected.
+    {
+        const HeapEntry u = side.open_pop(S, 2 * H, lane, WL);
+        const bool stop = max_iter <= 0 || u.v < 0 || u.k >= side.worst_of(S);
+        if (lane == 0) {
+            ctl->pop_u[0] = stop ? -1 : u.v;
+            ctl->root_k[0] = S.open[1].k;
+            ctl->root_v[0] = S.open[1].v;
+            ctl->guess[0] = ctl->guess[1] = -2;
+        }
+    }
+    PA_TICK(2);
+    for (int step = 0; step < max_iter; ++step) {
+        const int p = step & 1;
+        cta_sync();
+        PA_TICK(4);
+        const int u = ctl->pop_u[p];
+        if (u < 0) break;
+        if (u != ctl->guess[p]) cta_sync();  // the gather warps fetch node u now
+        PA_TICK(3);
+        // heap_update (:23-39) in row order, then the next pop (:84-90)
+        const int n_new = ctl->n_new[p];
+        count_expansion(st, n_new, lane);
+        side.admit(S, S.nb_id + p * kMaxDegree, S.nb_d + p * kMaxDegree, n_new, log_room, H, lane,
+                   WL, ctl, [&](float dist, int32_t id, int) {
+                       side.open_push(S, 2 * H, dist, id, lane, WL);
+#if PA_REFINE_PROFILE
+                       if (PA_REFINE_PROFILE == 1 && threadIdx.x == 0) prof[7] += 1;
+#endif
+                   });
+        PA_TICK(5);
+        if (step + 1 < max_iter) {
+            const HeapEntry nx = side.open_pop(S, 2 * H, lane, WL);
+            const bool stop = nx.v < 0 || nx.k >= side.worst_of(S);
+            if (lane == 0) {
+                ctl->pop_u[p ^ 1] = stop ? -1 : nx.v;
+                ctl->root_k[p ^ 1] = S.open[1].k;
+                ctl->root_v[p ^ 1] = S.open[1].v;
+            }
+        }
+        PA_TICK(2);
+    }
+}
+
+// The heap warp's half of a stage.  Out of line: the registers of its heaps and those
+// of the gather's row loads are never live together, and inlined they were allocated as
+// if they were (rows spilled, 768 dimensions 17.8 instead of 16.1 ms per 8192 queries).
+template <int R>
+__device__ __noinline__ void heap_side(const RefineArgs &A, RefCtl *ctl, int n_seed, int max_iter,
+                                       bool second, bool brief, bool closed_form, int *st) {
+    const RefShared S = ref_shared(A, ref_smem);
+    const int lane = threadIdx.x & 31, H = A.H;
+    const int seed_lo = second ? max(n_seed - H, 0) : 0;
+    const WalkLane WL = walk_lane(lane);
+    HeapSide<R> side;
+    side.clear(H, lane);
+    ctl->amb = CUDART_INF_F;  // all lanes alike
+    st[0] = st[1] = 0;
+    __syncwarp();
+    int prof[12] = {};
+    long long prof_t = 0;
+    if (brief)
+        brief_search<R>(A, S, n_seed, ctl, side, WL, lane, st);
+    else
+        heap_loop<R>(A, S, n_seed, seed_lo, max_iter, closed_form, second ? H + seed_lo : 0, ctl,
+                     side, WL, lane, st, prof, prof_t);
+    side.finish(second ? S.open + H + 1 : S.buf + 1, H, lane, ctl);
+}
+
+// The gather warps' half of the general search.
+__device__ __forceinline__ void gather_loop(const RefineArgs &A, const RefShared &S,
+                                            const RefGraph &G, uint8_t *vis, uint8_t marker,
+                                            int max_iter, bool speculate, RefCtl *ctl, int gw,
+                                            int lane, int *prof, long long &prof_t) {
+    for (int step = 0; step < max_iter; ++step) {
+        const int p = step & 1;
+        cta_sync();
+        if (step == 0) { PA_GTICK(7); } else { PA_GTICK(6); }  // waiting for the heap warp: seed inserts / a pop
+        const int u = ctl->pop_u[p];
+        if (u < 0) break;
+        if (u != ctl->guess[p]) {  // CTA-uniform: nothing, or something else, was prepared
+            gather_node(A, S, G, vis, marker, ctl, u, p, gw, lane, prof, prof_t);
+            cta_sync();
+        }
+        if (speculate && step + 1 < max_iter) {
+            // the node the next pop returns unless it ends the search: the first
+            // new neighbour with the smallest distance if that is below the root
+            // the open heap had after this expansion's pop, else that root.
+            // Distances are sums of squares: their bits order like their values.
+            const int n_new = ctl->n_new[p];
+            const float *nb_d = S.nb_d + p * kMaxDegree;
+            unsigned best = __float_as_uint(CUDART_INF_F);
+            int at = 0;
+            for (int c = 0; c < n_new; c += 32) {
+                const unsigned key = c + lane < n_new ? __float_as_uint(nb_d[c + lane]) : ~0u;
+                const unsigned least = __reduce_min_sync(kAll, key);
+                if (least < best) {
+                    best = least;
+                    at = c + __ffs(__ballot_sync(kAll, key == least)) - 1;
+                }
+            }
+            const int guess = __uint_as_float(best) < ctl->root_k[p] ? S.nb_id[p * kMaxDegree + at]
+                                                                     : ctl->root_v[p];
+            if (gw == 0 && lane == 0) ctl->guess[p ^ 1] = guess;
+            if (guess >= 0) gather_node(A, S, G, vis, marker, ctl, guess, p ^ 1, gw, lane, prof, prof_t);
+        }
+    }
+}
+
+// Upstream's sequence at the end of a stage (:139-162), by the heap warp.
+template <int R>
+__device__ __noinline__ void upstream_output(const RefineArgs &A, const RefCtl *ctl, int n_seed,
+                                             int n_real, int k_out, bool second) {
+    constexpr int kReplayWords = R >= 4 ? R / 2 : 1;
+    const RefShared S = ref_shared(A, ref_smem);
+    const int lane = threadIdx.x & 31, H = A.H;
+    const int seed_lo = second ? max(n_seed - H, 0) : 0;
+    PathBits<kReplayWords> smaller;
+    const WalkLane WL = walk_lane(lane);
+    auto push = [&](float dist, int32_t id) {
+        if (R == 0) warp_pushpop(S.buf, H, -dist, id, lane, WL);
+        else if (!(-dist <= S.buf[1].k))
+            bit_sink(S.buf, H, HeapEntry{-dist, id}, smaller, lane);
+    };
+    auto pop = [&]() {
+        if (R == 0) return warp_pop(S.buf, H, lane, WL);
+        const HeapEntry out = S.buf[1];
+        __syncwarp();
+        bit_sink(S.buf, H, HeapEntry{CUDART_INF_F, -1}, smaller, lane);
+        return out;
+    };
+    if (R > 0) {
+        // the result heap as upstream's pushes leave it; the log's part in buf makes
+        // room for it by going where the list was
+        HeapEntry *moved = S.open;
+        const int n_log = second ? ctl->n_log : 0, in_buf = min(n_log, H);
+        for (int i = lane; i < in_buf; i += 32) moved[i] = S.buf[1 + i];
+        __syncwarp();
+        for (int i = lane; i < H + 2; i += 32) S.buf[i] = HeapEntry{-CUDART_INF_F, -1};
+        smaller.clear();
+        __syncwarp();
+        for (int i = 0; i < n_log; ++i) {
+            const HeapEntry e = i < H ? moved[i] : HeapEntry{S.c_d[i - H], S.c_id[i - H]};
+            push(e.k, e.v);
+        }
+        for (int x = 0; !second && x < ctl->st[0]; ++x)  // the expansions of the first stage
+            for (int j = 0; j < ctl->n_new[x]; ++j) {
+                const float dist = S.nb_d[x * kMaxDegree + j];
+                if (!(dist >= -S.buf[1].k)) push(dist, S.nb_id[x * kMaxDegree + j]);
+            }
+    }
+    for (int i = seed_lo; i < n_seed; ++i) {
+        const int id = S.c_id[i];
+        if (id >= 0) push(S.c_d[i], id);
+    }
+    for (int i = k_out; i < H; ++i) pop();
+    // what is left, worst first, into the open heap's memory: the seeds are in use
+    for (int i = 0; i < n_real; ++i) {
+        const HeapEntry e = pop();
+        if (lane == 0) S.open[H + 1 - i] = HeapEntry{-e.k, e.v};
+    }
+    __syncwarp();
+    for (int i = lane; i < n_real; i += 32) {
+        const HeapEntry e = S.open[H + 2 - n_real + i];
+        S.c_id[k_out - n_real + i] = e.v;
+        S.c_d[k_out - n_real + i] = e.k;
+    }
 }
 
 // One call of upstream's traverse_cpu_kernel: seeds in c_id / c_d (n_seed of
 // them), the result (k_out entries, ascending behind (-1, -inf) pads) back into
 // c_id / c_d.  `from` < d: the seeds' distances are first completed over dims
-// [from, d).  Returns expansions and evaluations through n_expand / n_eval
-// (warp 0).
-__device__ __forceinline__ void search_stage(const RefineArgs &A, const RefShared &S,
+// [from, d).  `second`: the full-graph stage behind the sub-graph stage, whose seeds
+// are that stage's output.  n_check: how many leading entries of the output have to be
+// upstream's in the order of equal distances, too.  Returns expansions and
+// evaluations through ctl->st, and false (CTA-uniform) if the query
+// has to be run on the array heaps (R > 0 only: a NaN distance, which upstream's tests
+// let into the heaps, or equal distances after more admissions than the log holds).
+template <int R>
+__device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShared &S,
                                              const RefGraph &G, uint8_t *vis, uint8_t marker,
                                              int n_seed, int from, int max_iter, int k_out,
-                                             bool speculate, bool seeds_sorted, RefCtl *ctl,
-                                             int &n_expand, int &n_eval, int *prof,
+                                             bool second, int n_check, RefCtl *ctl, int *prof,
                                              long long &prof_t) {
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int d = A.d, H = A.H;
+    const bool speculate = second;
     (void)prof; (void)prof_t;
     // distances completed over the trailing dims (:41-62), in place
     if (from < d) {
@@ -756,7 +1346,8 @@ __device__ __forceinline__ void search_stage(const RefineArgs &A, const RefShare
     }
     PA_GTICK(4);  // residual distances of the seeds
     // :65-68
-    for (int i = tid; i < H + 2; i += blockDim.x) S.buf[i] = HeapEntry{-CUDART_INF_F, -1};
+    if (R == 0)
+        for (int i = tid; i < H + 2; i += blockDim.x) S.buf[i] = HeapEntry{-CUDART_INF_F, -1};
     for (int i = tid; i < 2 * H + 2; i += blockDim.x) S.open[i] = HeapEntry{CUDART_INF_F, -1};
     // :69-79, the marks (their order does not matter; the heap inserts below keep it)
     for (int i = tid; i < n_seed; i += blockDim.x) {
@@ -765,133 +1356,56 @@ __device__ __forceinline__ void search_stage(const RefineArgs &A, const RefShare
     }
     __syncthreads();
     PA_TICK(0);
-    const WalkLane WL = walk_lane(lane);
+    // seeds of the second stage: behind the pads the first stage left
+    const int seed_lo = second ? max(n_seed - H, 0) : 0;
+    // Log of the second stage: H entries in buf, the others where its pads were; the list
+    // then goes behind the part of the open heap that the merge writes.  The first stage
+    // has no log: its neighbours are still in their buffers.
+    const int log_room = second ? H + seed_lo : 0;
+    HeapEntry *list = second ? S.open + H + 1 : S.buf + 1;
+    const int sorted = second ? ctl->sorted : 0;
     const bool brief = max_iter == 2 && !speculate && 2 * H >= 32 && G.degree <= 64 &&
-                       brief_search(A, S, G, vis, marker, n_seed, ctl, WL, n_expand, n_eval, prof, prof_t);
-    if (!brief && w == 0) {
-        if (seeds_sorted && ctl->sorted != 0 && n_seed >= H) {
-            // The real seeds are c[n_seed - H ..] in strictly ascending order.  Every
-            // key offered to heap_replace is then larger than all keys in the heap:
-            // it replaces a +inf leaf and climbs to just below a real entry, or meets
-            // a real leaf and is dropped -- which of the two depends on the count of
-            // seeds before it only.  Seed 0 ends at heap index 0, seeds 2t - 1 and 2t
-            // at the two rightmost nodes of level t (2^(t+1) - 3 and 2^(t+1) - 2,
-            // 0-based) while those exist; all later seeds are dropped.  Checked
-            // against heap_replace for every heap size and seed count on the host.
-            const int t = (lane + 1) >> 1;
-            const int pos = lane == 0 ? 0 : (1 << (t + 1)) - 3 + ((lane & 1) ? 0 : 1);
-            const int at = n_seed - H + lane;
-            if (lane < 25 && pos < 2 * H && at < n_seed && S.c_id[at] >= 0)
-                S.open[1 + pos] = HeapEntry{S.c_d[at], S.c_id[at]};
-            __syncwarp();
-        } else {
-            for (int i = 0; i < n_seed; ++i) {
-                const int id = S.c_id[i];
-                if (id >= 0) warp_replace(S.open, 2 * H, S.c_d[i], id, lane, WL);
+                       brief_prepare(S, n_seed, ctl);
+    if (w == 0) {
+        heap_side<R>(A, ctl, n_seed, max_iter, second, brief,
+                     sorted == (kAscending | kHeadStrict) && n_seed >= H, ctl->st + (second ? 2 : 0));
+    } else if (brief) {
+        if (ctl->m1 != ~0ull) {
+            gather_node(A, S, G, vis, marker, ctl, S.c_id[ctl->m1 & 0xffffffffu], 0, w - 1, lane, prof, prof_t);
+            cta_sync();
+            cta_sync();  // the heap warp has the second node
+            const int u2 = ctl->pop_u[1];
+            if (u2 >= 0) {
+                gather_node(A, S, G, vis, marker, ctl, u2, 1, w - 1, lane, prof, prof_t);
+                cta_sync();
             }
         }
+    } else {
+        gather_loop(A, S, G, vis, marker, max_iter, speculate, ctl, w - 1, lane, prof, prof_t);
     }
-    PA_TICK(1);
-    // :82-136.  Expansion i uses slot i & 1 of the control block and of the
-    // neighbour buffers.  Per expansion one CTA-wide barrier: behind it the heap
-    // warp has popped node i (or ended the search) and -- when speculating --
-    // the gather warps have prepared the node they expected.
-    if (!brief && w == 0) {
-        const HeapEntry u = warp_pop(S.open, 2 * H, lane, WL);
-        const bool stop = max_iter <= 0 || u.v < 0 || u.k >= -S.buf[1].k;
-        if (lane == 0) {
-            ctl->pop_u[0] = stop ? -1 : u.v;
-            ctl->root_k[0] = S.open[1].k;
-            ctl->root_v[0] = S.open[1].v;
-            ctl->guess[0] = ctl->guess[1] = -2;
-        }
-    }
-    PA_TICK(2);
-    for (int step = 0; step < max_iter && !brief; ++step) {
-        const int p = step & 1;
-        __syncthreads();
-        PA_TICK(4);
-        if (step == 0) { PA_GTICK(7); } else { PA_GTICK(6); }  // waiting for the heap warp: seed inserts / a pop
-        const int u = ctl->pop_u[p];
-        if (u < 0) break;
-        if (u != ctl->guess[p]) {  // CTA-uniform: nothing, or something else, was prepared
-            if (w > 0) gather_node(A, S, G, vis, marker, ctl, u, p, w - 1, lane, prof, prof_t);
-            __syncthreads();
-        }
-        PA_TICK(3);
-        if (w == 0) {
-            // heap_update (:23-39) in row order, then the next pop (:84-90)
-            const int n_new = ctl->n_new[p];
-            const int32_t *nb_id = S.nb_id + p * kMaxDegree;
-            const float *nb_d = S.nb_d + p * kMaxDegree;
-            ++n_expand;
-            n_eval += n_new;
-            for (int j = 0; j < n_new; ++j) {
-                const float dist = nb_d[j];
-                if (dist >= -S.buf[1].k) continue;
-                warp_pushpop(S.buf, H, -dist, nb_id[j], lane, WL);
-                warp_replace(S.open, 2 * H, dist, nb_id[j], lane, WL);
-#if PA_REFINE_PROFILE
-                if (PA_REFINE_PROFILE == 1 && threadIdx.x == 0) prof[7] += 1;
-#endif
-            }
-            PA_TICK(5);
-            if (step + 1 < max_iter) {
-                const HeapEntry nx = warp_pop(S.open, 2 * H, lane, WL);
-                const bool stop = nx.v < 0 || nx.k >= -S.buf[1].k;
-                if (lane == 0) {
-                    ctl->pop_u[p ^ 1] = stop ? -1 : nx.v;
-                    ctl->root_k[p ^ 1] = S.open[1].k;
-                    ctl->root_v[p ^ 1] = S.open[1].v;
-                }
-            }
-            PA_TICK(2);
-        } else if (speculate && step + 1 < max_iter) {
-            // the node the next pop returns unless it ends the search: the first
-            // new neighbour with the smallest distance if that is below the root
-            // the open heap had after this expansion's pop, else that root
-            const int n_new = ctl->n_new[p];
-            const float *nb_d = S.nb_d + p * kMaxDegree;
-            float best = CUDART_INF_F;
-            int at = 0x7fffffff;
-            for (int j = lane; j < n_new; j += 32) {
-                const float dist = nb_d[j];
-                if (dist < best) { best = dist; at = j; }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                const float ob = __shfl_xor_sync(kAll, best, off);
-                const int oa = __shfl_xor_sync(kAll, at, off);
-                if (ob < best || (ob == best && oa < at)) { best = ob; at = oa; }
-            }
-            const int guess = best < ctl->root_k[p] ? S.nb_id[p * kMaxDegree + at] : ctl->root_v[p];
-            if (tid == 32) ctl->guess[p ^ 1] = guess;
-            if (guess >= 0) gather_node(A, S, G, vis, marker, ctl, guess, p ^ 1, w - 1, lane, prof, prof_t);
-        }
-        PA_TICK(5);
-    }
-    // :139-162: the seeds join the result heap; all but k_out are dropped; what is
+    __syncthreads();
+    if (R > 0 && (ctl->rerun != 0 || (second && (sorted & kAscending) == 0))) return false;
+    PA_TICK(5);
+    // :139-162: the seeds join the results; all but k_out are dropped; what is
     // left comes out worst first and is stored ascending
     const int n_real = min(k_out, H);
-    const bool sorted = select_sort_output(S, H, n_seed, n_real, k_out, ctl);  // CTA-uniform
-    if (tid == 0) ctl->sorted = sorted;  // the output is strictly ascending up to its trailing pads
-    if (!sorted) {
-        if (w == 0) {
-            for (int i = 0; i < n_seed; ++i) {
-                const int id = S.c_id[i];
-                if (id >= 0) warp_pushpop(S.buf, H, -S.c_d[i], id, lane, WL);
-            }
-            for (int i = k_out; i < H; ++i) warp_pop(S.buf, H, lane, WL);
-        }
-        __syncthreads();  // the seeds have been read: their slots may be overwritten
-        if (w == 0) {
-            for (int i = 0; i < n_real; ++i) {
-                const HeapEntry e = warp_pop(S.buf, H, lane, WL);
-                if (lane == 0) {
-                    S.c_id[k_out - i - 1] = e.v;
-                    S.c_d[k_out - i - 1] = -e.k;
-                }
-            }
+    const bool done =  // CTA-uniform
+        R > 0 && second
+            ? merge_sorted_output(S, list, H, seed_lo, n_seed, n_real, k_out, ctl)
+            : select_sort_output<R>(S, H, seed_lo, n_seed, n_real, k_out, min(n_check, n_real), ctl);
+    if (tid == 0) ctl->sorted = kAscending | kHeadStrict;  // select_sort_output has seen to it
+    if (!done) {
+        if (R > 0 && second && ctl->n_log > log_room) return false;
+        if (w == 0) upstream_output<R>(A, ctl, n_seed, n_real, k_out, second);
+        __syncthreads();
+        // NaN distances may come out in any order; equal ones near the front forbid the
+        // closed form of the next stage's seeding (pads are not seeded)
+        for (int i = tid; i + 1 < n_real; i += blockDim.x) {
+            const int at = k_out - n_real + i;
+            if (!(S.c_d[at] <= S.c_d[at + 1])) ctl->sorted = 0;
+            else if (i < kSeedHead && S.c_d[at] == S.c_d[at + 1] &&
+                     (S.c_id[at] >= 0 || S.c_id[at + 1] >= 0))
+                atomicAnd(&ctl->sorted, kAscending);
         }
     }
     // pops of an exhausted heap give (-1, key +inf): the leading pads
@@ -902,21 +1416,88 @@ __device__ __forceinline__ void search_stage(const RefineArgs &A, const RefShare
     __syncthreads();
     PA_TICK(6);
     PA_GTICK(8);  // merge and output
+    return true;
 }
 
-__global__ void __launch_bounds__(kRefThreads, PA_REFINE_MIN_CTAS) refine_kernel(RefineArgs A) {
-    extern __shared__ __align__(16) unsigned char ref_smem[];
+// Query b from its candidates to its output.  False: see search_stage.
+template <int R>
+__device__ __forceinline__ bool run_query(const RefineArgs &A, const RefShared &S, int64_t b,
+                                          int slot, uint8_t *vis, RefCtl *ctl) {
+    const int tid = threadIdx.x;
+    // next marker of this slot; the array is wiped when the markers run out
+    // (bitmask.hpp:17-36 does the same on wrap-around)
+    if (tid == 0) {
+        ctl->marker = A.epoch[slot] + 1;
+        ctl->rerun = 0;
+        ctl->st[2] = ctl->st[3] = 0;
+    }
+    __syncthreads();
+    int marker = ctl->marker;
+    if (marker > 254) {
+        uint4 *p = reinterpret_cast<uint4 *>(vis);
+        for (int64_t i = tid; i < A.slot_stride / 16; i += blockDim.x)
+            p[i] = make_uint4(0, 0, 0, 0);
+        marker = 1;
+    }
+    __syncthreads();
+    if (tid == 0) A.epoch[slot] = marker;
+
+    for (int i = tid; i < A.d; i += blockDim.x) S.q[i] = A.query[b * A.ldq + i];
+    for (int i = tid; i < A.n_cand; i += blockDim.x) {
+        const int64_t id = A.cand_I[b * A.n_cand + i];
+        S.c_id[i] = (id < 0 || id >= A.n_nodes) ? -1 : static_cast<int32_t>(id);
+        S.c_d[i] = A.cand_D[b * A.n_cand + i];
+    }
+    __syncthreads();
+    int prof[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    long long prof_t = 0;
+#if PA_REFINE_PROFILE
+    prof_t = pinned_clock();
+#endif
+    // stage 2 (traverse_cpu.cpp:317-326): sub-graph, REFINE_STEP expansions
+    const int k_last = A.stages >= 3 ? A.k : A.n_cand;
+    if (!search_stage<R>(A, S, A.sub, vis, static_cast<uint8_t>(marker), A.n_cand, A.d_p,
+                         min(2, 2 * A.ef), A.n_cand, false, A.stages >= 3 ? max(A.k, kSeedHead) : A.H,
+                         ctl, prof, prof_t))
+        return false;
+    if (A.stages >= 3 &&  // stage 3 (:327-336): full graph, same marker
+        !search_stage<R>(A, S, A.full, vis, static_cast<uint8_t>(marker), A.n_cand, A.d,
+                         min(1024, 2 * A.ef), A.k, true, A.k, ctl, prof, prof_t))
+        return false;
+    for (int i = tid; i < k_last; i += blockDim.x) {
+        A.out_I[b * k_last + i] = S.c_id[i];
+        A.out_D[b * k_last + i] = S.c_d[i];
+    }
+#if PA_REFINE_PROFILE
+    if (A.stats != nullptr && tid == 32)
+        for (int i = 0; i < 12; ++i) A.stats[b * 24 + 12 + i] = prof[i];
+#endif
+    if (A.stats != nullptr && tid == 0) {
+#if PA_REFINE_PROFILE
+        for (int i = 0; i < 4; ++i) A.stats[b * 24 + i] = ctl->st[i];
+        for (int i = 0; i < 8; ++i) A.stats[b * 24 + 4 + i] = prof[i];
+#else
+#pragma unroll
+        for (int i = 0; i < 4; ++i) A.stats[b * 4 + i] = ctl->st[i];
+#endif
+    }
+    return true;
+}
+
+// The way back to the array heaps, out of line: it has hardly ever work to do.
+__device__ __noinline__ void run_query_again(const RefineArgs &A, int64_t b, RefCtl *ctl) {
+    __syncthreads();
+    const RefShared S = ref_shared(A, ref_smem);
+    const int slot = A.slot_begin + blockIdx.x;
+    run_query<0>(A, S, b, slot, A.marks + static_cast<int64_t>(slot) * A.slot_stride, ctl);
+}
+
+template <int R>
+__global__ void __launch_bounds__(kRefThreads, PA_REFINE_MIN_CTAS)
+refine_kernel(const __grid_constant__ RefineArgs A) {
     __shared__ RefCtl ctl_s;
     RefCtl *ctl = &ctl_s;
-    RefShared S;
-    S.q = reinterpret_cast<float *>(ref_smem);
-    S.open = reinterpret_cast<HeapEntry *>(S.q + A.d);
-    S.buf = S.open + 2 * A.H + 2;
-    S.c_id = reinterpret_cast<int32_t *>(S.buf + A.H + 2);
-    S.c_d = reinterpret_cast<float *>(S.c_id + A.n_cand);
-    S.nb_id = reinterpret_cast<int32_t *>(S.c_d + A.n_cand);
-    S.nb_d = reinterpret_cast<float *>(S.nb_id + 2 * kMaxDegree);
-    S.stage = S.nb_d + 2 * kMaxDegree;
+    const RefShared S = ref_shared(A, ref_smem);
     const int tid = threadIdx.x;
     const int slot = A.slot_begin + blockIdx.x;
     uint8_t *vis = A.marks + static_cast<int64_t>(slot) * A.slot_stride;
@@ -924,59 +1505,7 @@ __global__ void __launch_bounds__(kRefThreads, PA_REFINE_MIN_CTAS) refine_kernel
     // CTA i starts on query i; whoever finishes claims the next unclaimed query (queries
     // differ several-fold in length, and a launch is over when its last CTA is)
     for (int64_t b = blockIdx.x; b < A.batch;) {
-        // next marker of this slot; the array is wiped when the markers run out
-        // (bitmask.hpp:17-36 does the same on wrap-around)
-        if (tid == 0) ctl->marker = A.epoch[slot] + 1;
-        __syncthreads();
-        int marker = ctl->marker;
-        if (marker > 254) {
-            uint4 *p = reinterpret_cast<uint4 *>(vis);
-            for (int64_t i = tid; i < A.slot_stride / 16; i += blockDim.x)
-                p[i] = make_uint4(0, 0, 0, 0);
-            marker = 1;
-        }
-        __syncthreads();
-        if (tid == 0) A.epoch[slot] = marker;
-
-        for (int i = tid; i < A.d; i += blockDim.x) S.q[i] = A.query[b * A.ldq + i];
-        for (int i = tid; i < A.n_cand; i += blockDim.x) {
-            const int64_t id = A.cand_I[b * A.n_cand + i];
-            S.c_id[i] = (id < 0 || id >= A.n_nodes) ? -1 : static_cast<int32_t>(id);
-            S.c_d[i] = A.cand_D[b * A.n_cand + i];
-        }
-        __syncthreads();
-        int st[4] = {0, 0, 0, 0};
-        int prof[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-        long long prof_t = 0;
-#if PA_REFINE_PROFILE
-        prof_t = pinned_clock();
-#endif
-        // stage 2 (traverse_cpu.cpp:317-326): sub-graph, REFINE_STEP expansions
-        search_stage(A, S, A.sub, vis, static_cast<uint8_t>(marker), A.n_cand, A.d_p,
-                     min(2, 2 * A.ef), A.n_cand, false, false, ctl, st[0], st[1], prof, prof_t);
-        int k_out = A.n_cand;
-        if (A.stages >= 3) {  // stage 3 (:327-336): full graph, same marker
-            search_stage(A, S, A.full, vis, static_cast<uint8_t>(marker), A.n_cand, A.d,
-                         min(1024, 2 * A.ef), A.k, true, true, ctl, st[2], st[3], prof, prof_t);
-            k_out = A.k;
-        }
-        for (int i = tid; i < k_out; i += blockDim.x) {
-            A.out_I[b * k_out + i] = S.c_id[i];
-            A.out_D[b * k_out + i] = S.c_d[i];
-        }
-#if PA_REFINE_PROFILE
-        if (A.stats != nullptr && tid == 32)
-            for (int i = 0; i < 12; ++i) A.stats[b * 24 + 12 + i] = prof[i];
-#endif
-        if (A.stats != nullptr && tid == 0) {
-#if PA_REFINE_PROFILE
-            for (int i = 0; i < 4; ++i) A.stats[b * 24 + i] = st[i];
-            for (int i = 0; i < 8; ++i) A.stats[b * 24 + 4 + i] = prof[i];
-#else
-#pragma unroll
-            for (int i = 0; i < 4; ++i) A.stats[b * 4 + i] = st[i];
-#endif
-        }
+        if (!run_query<R>(A, S, b, slot, vis, ctl)) run_query_again(A, b, ctl);
         if (tid == 0) ctl->next = atomicAdd(A.claim, 1u);
         __syncthreads();
         b = static_cast<int64_t>(gridDim.x) + ctl->next;
@@ -998,24 +1527,34 @@ int refine_ctas_per_sm(int d_model) {
     return by_registers < 12 ? by_registers : 12;  // shared memory: about 17 KB per CTA
 }
 
+// one staged row per warp: a narrow CTA may be launched with up to four warps
+static int ref_stage_rows(int d) { return max(ref_threads_for(d), 128) / 32; }
+
 static size_t refine_smem_bytes(int d, int H, int n_cand) {
-    // one staged row per warp: a narrow CTA may be launched with up to four warps
-    const int warps = max(ref_threads_for(d), 128) / 32;
-    return sizeof(float) * d * (1 + warps) + sizeof(HeapEntry) * (3 * H + 4) +
+    return sizeof(float) * d * (1 + ref_stage_rows(d)) + sizeof(HeapEntry) * (3 * H + 4) +
            8 * static_cast<size_t>(n_cand) + 16 * kMaxDegree;
+}
+
+template <int R>
+static int refine_launch_with(const RefineArgs &A, unsigned grid, int threads, int dev,
+                              cudaStream_t stream) {
+    const size_t smem = refine_smem_bytes(A.d, A.H, A.n_cand);
+    static size_t configured[64] = {};
+    if (smem > 48 * 1024 && dev >= 0 && dev < 64 && configured[dev] < smem) {
+        PA_CUDA_TRY(cudaFuncSetAttribute(refine_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem)));
+        configured[dev] = smem;
+    }
+    refine_kernel<R><<<grid, threads, smem, stream>>>(A);
+    count_launch();
+    PA_CUDA_TRY(cudaGetLastError());
+    return PA_OK;
 }
 
 static int refine_launch(const RefineArgs &A, int n_slots, cudaStream_t stream) {
     if (A.batch == 0) return PA_OK;
-    const size_t smem = refine_smem_bytes(A.d, A.H, A.n_cand);
-    static size_t configured[64] = {};
     int dev = 0;
     PA_CUDA_TRY(cudaGetDevice(&dev));
-    if (smem > 48 * 1024 && dev >= 0 && dev < 64 && configured[dev] < smem) {
-        PA_CUDA_TRY(cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem)));
-        configured[dev] = smem;
-    }
     const unsigned grid = static_cast<unsigned>(min(static_cast<int64_t>(A.batch),
                                                     static_cast<int64_t>(n_slots)));
     int threads = ref_threads_for(A.d);
@@ -1027,10 +1566,12 @@ static int refine_launch(const RefineArgs &A, int n_slots, cudaStream_t stream) 
             if (grid <= 9u * static_cast<unsigned>(sms[dev])) threads = 128;
         }
     }
-    refine_kernel<<<grid, threads, smem, stream>>>(A);
-    count_launch();
-    PA_CUDA_TRY(cudaGetLastError());
-    return PA_OK;
+    switch (list_regs_for(A.H)) {
+        case 2: return refine_launch_with<2>(A, grid, threads, dev, stream);
+        case 4: return refine_launch_with<4>(A, grid, threads, dev, stream);
+        case 8: return refine_launch_with<8>(A, grid, threads, dev, stream);
+        default: return refine_launch_with<0>(A, grid, threads, dev, stream);
+    }
 }
 
 static int refine_check(const void *out_I, const void *out_D, const void *cand_I, const void *cand_D,

@@ -353,6 +353,61 @@ def test_equal_distances_take_upstreams_sequence(oracle_lib):
         assert row.unique().numel() < row.numel()
 
 
+@pytest.mark.parametrize("ef,k,spoil", [(16, 16, None), (30, 10, "pairs"), (48, 48, "pairs"),
+                                        (64, 10, "nan"), (96, 90, "pairs"), (128, 100, "pairs"),
+                                        (150, 10, "nan"), (192, 100, "pairs"), (256, 200, "pairs"),
+                                        (257, 20, "pairs")])
+def test_result_list_of_every_capacity(oracle_lib, ef, k, spoil):
+    """Every capacity of the result list in registers (16 .. 256, the next one has the
+    array heaps), with long results; "pairs": some vectors twice, so that a few equal
+    distances reach the merges and the log of admissions is replayed; "nan": a vector
+    of NaN that searches meet, which sends the query back to the array heaps.  Bit for
+    bit the oracle's, statistics included (with NaN, which the heaps do not order, for the
+    queries that do not meet one)."""
+    from pilotann_b200 import extension
+    from helpers import make_problem
+    B, n, d, d_p = 40, 4000, 48, 16
+    g = torch.Generator().manual_seed(1000 + ef)
+    p = make_problem(n=n, d=d, ratio=0.5, batch=B, n_init=32, seed=700)
+    full, q = p["full"].clone(), p["query"]
+    if spoil == "pairs":
+        twins = torch.randperm(n, generator=g)[:400].view(2, -1)
+        full[twins[0]] = full[twins[1]]
+    ids = p["nodelist"][torch.randint(p["nodelist"].numel(), (B, 4 * ef), generator=g)]
+    if spoil == "nan":
+        # a neighbour of the first candidates, itself no candidate
+        bad = p["full_indices"][p["full_indptr"][ids[::8, 0]]].unique()
+        full[bad] = float("nan")
+        keep = ids[~torch.isin(ids, bad)]
+        ids = keep[torch.randint(keep.numel(), (B, 4 * ef), generator=g)]
+    dist = ((q[:, :d_p].unsqueeze(1) - full[ids][:, :, :d_p]) ** 2).sum(-1).contiguous()
+    nbr, row_of = extension.pack_graph(p["indptr"].cuda(), p["indices"].cuda(), p["mapping"].cuda(),
+                                       p["storage"].size(0), 32)
+    full_nbr = extension.pack_fullgraph(p["full_indptr"].cuda(), p["full_indices"].cuda(), 32)
+    pool = extension.VisitedPool(n, 16)
+    graphs = ([p["indptr"], p["indices"]], [p["full_indptr"], p["full_indices"]])
+    for top in (None, k):
+        st = torch.zeros(B, 4, dtype=torch.int32, device="cuda")
+        t_I, t_D = extension.refine(ids.cuda(), dist.cuda(), q.cuda(), full.cuda(), nbr, row_of,
+                                    full_nbr, pool, ef, d_p, k=top, stats=st)
+        torch.cuda.synchronize()
+        w_bI, w_bD = ids.clone(), dist.clone()
+        w_I, w_D, w_st = oracle_lib.refine_ex(w_bI, w_bD, *graphs, full, q, k, ef, d_p, gpu_order=True,
+                                              stages=3 if top else 2, with_stats=True)
+        if top is None:
+            w_I, w_D, w_st, st = w_bI, w_bD, w_st[:, :2], st[:, :2]
+        if spoil == "nan":
+            same = (t_I.cpu() == w_I).all(1) & (t_D.cpu() == w_D).all(1) & (st.cpu() == w_st).all(1)
+            assert 0.2 < same.float().mean() and ((t_I >= -1) & (t_I < n)).all(), top
+            again = extension.refine(ids.cuda(), dist.cuda(), q.cuda(), full.cuda(), nbr, row_of,
+                                     full_nbr, pool, ef, d_p, k=top)
+            assert torch.equal(again[0], t_I)
+            continue
+        assert torch.equal(t_I.cpu(), w_I), top
+        assert torch.equal(t_D.cpu().view(torch.int32), w_D.view(torch.int32)), top
+        assert torch.equal(st.cpu(), w_st), top
+
+
 def test_replay_of_upstream_fixtures():
     """Outputs of upstream ``traverse_refine`` recorded by tests/golden/make_golden.py
     (CPU, no GPU involved), replayed through the refinement kernel without the
