@@ -45,6 +45,7 @@
 //                   computed when the index is packed: two dependent loads per
 //                   hop (neighbour row, vector rows) and no hashing in the loop.
 #include "pa_common.cuh"
+#include "warp_heap.cuh"
 
 namespace pa {
 
@@ -426,6 +427,62 @@ __device__ __forceinline__ float list_at(const float (&cd)[4], unsigned p) {
     return __shfl_sync(kFull, mine, p & 7u, kGroup);
 }
 
+// distances (traverse_cuda.cu:187-204) by teams of 8 lanes, two candidates in flight per
+// team: team `team` of `n_teams` takes candidates j_begin + team,
+// + n_teams, ... below j_end.  The loop bound is the same for every lane of
+// a warp (the team shuffles name the whole warp); lanes past the end carry
+// a false predicate.  `spare`: 32 slots behind the candidates, one per lane.
+        template <class Layout>
+__device__ __forceinline__ void team_distances(const Layout &L, int2 *slots, float *cand_d,
+                                               int spare, const float *q_s, int d, int lane,
+                                               int team, int n_teams, int j_begin, int j_end) {
+            const int t8 = lane & 7;
+            for (int jb = j_begin; jb < j_end; jb += 2 * n_teams) {
+                const int j0 = jb + team;
+                const int j1 = j0 + n_teams;
+                const bool p0_in = j0 < j_end, p1_in = j1 < j_end;
+                // Lanes past the end or without a vector read row 0 and drop the
+                // result: every load below is unconditional, no lane-dependent branch.
+                // (j0, j1 stay inside the arrays: they are below j_end + 2 * n_teams.)
+                int2 s0 = slots[j0], s1 = slots[j1];
+                if constexpr (!Layout::kPacked) {
+                    s0.y = static_cast<int32_t>(__ldg(L.mapping + (p0_in ? s0.x : 0)));
+                    s1.y = static_cast<int32_t>(__ldg(L.mapping + (p1_in ? s1.x : 0)));
+                    slots[(t8 == 0 && p0_in) ? j0 : spare + lane].y = s0.y;
+                    slots[(t8 == 0 && p1_in) ? j1 : spare + lane].y = s1.y;
+                }
+                const bool p0 = p0_in && s0.y >= 0, p1 = p1_in && s1.y >= 0;
+                const float *r0 = L.storage + static_cast<int64_t>(p0 ? s0.y : 0) * d;
+                const float *r1 = L.storage + static_cast<int64_t>(p1 ? s1.y : 0) * d;
+                float a0 = 0.0f, a1 = 0.0f;
+                for (int o = 4 * t8; o < d; o += 128) {
+                    // up to four stripes of each row in flight before any arithmetic
+                    float4 x0[4], x1[4];
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        const bool in = o + 32 * m < d;
+                        x0[m] = in ? __ldg(reinterpret_cast<const float4 *>(r0 + o + 32 * m))
+                                   : make_float4(0, 0, 0, 0);
+                        x1[m] = in ? __ldg(reinterpret_cast<const float4 *>(r1 + o + 32 * m))
+                                   : make_float4(0, 0, 0, 0);
+                    }
+#pragma unroll
+                    for (int m = 0; m < 4; ++m) {
+                        if (o + 32 * m < d) {
+                            const float4 qa = *reinterpret_cast<const float4 *>(q_s + o + 32 * m);
+                            a0 = stripe(a0, qa, x0[m]);
+                            a1 = stripe(a1, qa, x1[m]);
+                        }
+                    }
+                }
+                a0 = team_reduce(a0);
+                a1 = team_reduce(a1);
+                // +inf marks a candidate without a vector: it is never inserted
+                cand_d[(t8 == 0 && p0_in) ? j0 : spare + lane] = p0 ? a0 : CUDART_INF_F;
+                cand_d[(t8 == 0 && p1_in) ? j1 : spare + lane] = p1 ? a1 : CUDART_INF_F;
+            }
+        }
+
 template <int H, int CH, class Layout>
 __global__ void __launch_bounds__(kThreads, PA_MIN_CTAS)
 traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D,
@@ -709,57 +766,8 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
         const int n_work = n_work_s;
         if (n_work < kTeamsPerWarp) break;  // :182-184, uniform over the CTA
 
-        // distances (:187-204) by teams of 8 lanes, two candidates in flight per
-        // team: team `team` of `n_teams` takes candidates j_begin + team,
-        // + n_teams, ... below j_end.  The loop bound is the same for every lane of
-        // a warp (the team shuffles name the whole warp); lanes past the end carry
-        // a false predicate.
         auto distances = [&](int team, int n_teams, int j_begin, int j_end) {
-            const int t8 = lane & 7;
-            for (int jb = j_begin; jb < j_end; jb += 2 * n_teams) {
-                const int j0 = jb + team;
-                const int j1 = j0 + n_teams;
-                const bool p0_in = j0 < j_end, p1_in = j1 < j_end;
-                // Lanes past the end or without a vector read row 0 and drop the
-                // result: every load below is unconditional, no lane-dependent branch.
-                // (j0, j1 stay inside the arrays: they are below j_end + 2 * n_teams.)
-                int2 s0 = slots[j0], s1 = slots[j1];
-                if constexpr (!Layout::kPacked) {
-                    s0.y = static_cast<int32_t>(__ldg(L.mapping + (p0_in ? s0.x : 0)));
-                    s1.y = static_cast<int32_t>(__ldg(L.mapping + (p1_in ? s1.x : 0)));
-                    slots[(t8 == 0 && p0_in) ? j0 : kSpare + lane].y = s0.y;
-                    slots[(t8 == 0 && p1_in) ? j1 : kSpare + lane].y = s1.y;
-                }
-                const bool p0 = p0_in && s0.y >= 0, p1 = p1_in && s1.y >= 0;
-                const float *r0 = L.storage + static_cast<int64_t>(p0 ? s0.y : 0) * d;
-                const float *r1 = L.storage + static_cast<int64_t>(p1 ? s1.y : 0) * d;
-                float a0 = 0.0f, a1 = 0.0f;
-                for (int o = 4 * t8; o < d; o += 128) {
-                    // up to four stripes of each row in flight before any arithmetic
-                    float4 x0[4], x1[4];
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const bool in = o + 32 * m < d;
-                        x0[m] = in ? __ldg(reinterpret_cast<const float4 *>(r0 + o + 32 * m))
-                                   : make_float4(0, 0, 0, 0);
-                        x1[m] = in ? __ldg(reinterpret_cast<const float4 *>(r1 + o + 32 * m))
-                                   : make_float4(0, 0, 0, 0);
-                    }
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        if (o + 32 * m < d) {
-                            const float4 qa = *reinterpret_cast<const float4 *>(q_s + o + 32 * m);
-                            a0 = stripe(a0, qa, x0[m]);
-                            a1 = stripe(a1, qa, x1[m]);
-                        }
-                    }
-                }
-                a0 = team_reduce(a0);
-                a1 = team_reduce(a1);
-                // +inf marks a candidate without a vector: it is never inserted
-                cand_d[(t8 == 0 && p0_in) ? j0 : kSpare + lane] = p0 ? a0 : CUDART_INF_F;
-                cand_d[(t8 == 0 && p1_in) ? j1 : kSpare + lane] = p1 ? a1 : CUDART_INF_F;
-            }
+            team_distances(L, slots, cand_d, kSpare, q_s, d, lane, team, n_teams, j_begin, j_end);
         };
         const int count = deal_count(n_work, beam);  // length of this group's beam list
 
@@ -889,10 +897,34 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
     __syncthreads();
 
     // ---- store (:230-245): per beam worst -> best ----------------------------------
-    // The result warp pops into the rows of the open heaps' values, which are dead
-    // by now; all threads then write the output with coalesced stores.
+    // What the pops of upstream's result heap return, into the rows of the open heaps'
+    // values, which are dead by now; all threads then write the output with coalesced
+    // stores.  With pairwise different keys that is the heap in ascending order: warp b
+    // sorts beam b in registers.  Equal keys among the entries that come out: the layout
+    // of the heap decides, and the result warp pops them one by one, H dependent heap
+    // operations.  Popping always, 1024 queries took (us) 431, 1946 and 522 instead of 408,
+    // 1894 and 484 (96 dimensions at ef 256, 200 at 192, 2000 of 96 at 128).
     const int n_discard = max(H - ef, 0), n_real = min(ef, H);
-    if (w == 1) {
+    if (threadIdx.x == 0) again_s[0] = 0;
+    __syncthreads();
+    {
+        float k[H / 32];
+        int32_t v[H / 32];
+#pragma unroll
+        for (int e = 0; e < H / 32; ++e) {
+            k[e] = res_key[w][lane * (H / 32) + e];
+            v[e] = res_id[w][lane * (H / 32) + e];
+        }
+        warp_sort(k, v, lane);
+        if (warp_has_twins(k, v, n_discard, lane)) again_s[0] = 1;
+#pragma unroll
+        for (int e = 0; e < H / 32; ++e) {
+            const int i = lane * (H / 32) + e - n_discard;
+            if (i >= 0) open_val[w][i] = make_int2(v[e], __float_as_int(-k[e]));
+        }
+    }
+    __syncthreads();
+    if (w == 1 && again_s[0] != 0) {
         for (int p = 0; p < n_discard + n_real; ++p) {
             const float key = rkey[0];
             const int32_t id = rid[0];
