@@ -966,6 +966,331 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
     }
 }
 
+// ---- small batches: eight warps per query ------------------------------------------
+// The search above, operation for operation, for launches that leave the SMs room.  A
+// round is a chain -- pop, neighbour row, bloom filter, distances, inserts -- and with
+// few queries per SM its length is all that counts, so every beam has two warps of its
+// own: warp b drives the open heap of beam b (pop, neighbour row, heap_replace), warp
+// 4 + b its result heap, each with 32 lanes on one heap and the outcome of its
+// comparisons in registers (PathBits), so the eight heaps proceed side by side; all
+// eight warps evaluate distances, 64 candidates in one pass.  The bloom filter is one
+// sequence over the four rows and stays with warp 0.  What the next pop returns is
+// known before the inserts (the better of the open heap's root and the beam's best
+// candidate), so its neighbour row is on its way while they run.
+//
+// It takes three times the heap instructions of the kernel above, which keeps four
+// heaps in step in one warp, so it pays while an SM has one or two queries.  Search
+// without refinement, four warps / eight warps, us: 1 million vectors, 128 dimensions at
+// ef 128: 1 query 598 / 518, 148 835 / 641, 296 867 / 737, 444 899 / 882, 592 923 / 1005; 96
+// dimensions at ef 48: 148 263 / 236, 296 275 / 266, 444 298 / 329; 64 dimensions at ef 128
+// in clusters: 148 185 / 164, 296 197 / 208, 444 240 / 265.  Sixteen warps: 543, 623, 754 at
+// the first three sizes.
+constexpr int kWideThreads = 256;
+constexpr int kWidePerSm = 2;  // up to this many queries per SM
+
+__device__ __forceinline__ void beam_sync(int beam) {  // the two warps of a beam
+    asm volatile("bar.sync %0, 64;" ::"r"(beam + 1) : "memory");
+}
+
+template <int H, class Layout>
+__global__ void __launch_bounds__(kWideThreads, 4)
+traverse_wide_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D,
+                     const float *__restrict__ query, const int64_t *__restrict__ init_I,
+                     const float *__restrict__ init_D, int d, int64_t ldq, int n_init, int ef,
+                     int32_t *__restrict__ stats) {
+    constexpr int W = H <= 64 ? 1 : H / 64;
+    constexpr int n_nb = 32;
+    constexpr int kSpare = kBeams * n_nb;
+    __shared__ uint32_t bloom[kBloomWords];
+    // 1-based.  Open heap values: packed layout -- the storage row, -2 for a node without
+    // one; CSR layout -- the node; -1 marks an empty entry
+    __shared__ __align__(16) HeapEntry open_s[kBeams][H + 2];
+    __shared__ __align__(16) HeapEntry res_s[kBeams][H + 2];
+    __shared__ int2 row_s[kBeams * n_nb];     // a round's neighbour slots {id, storage row}
+    __shared__ uint2 probe_s[kBeams * n_nb];  // and their bloom probes
+    // survivors and their distances; team_distances looks at up to 64 entries past the
+    // last one, 32 of them are spare slots for stores that have nothing to write
+    __shared__ int2 slots[kBeams * n_nb + 64];
+    __shared__ float cand_d[kBeams * n_nb + 64];
+    __shared__ float worst_s[kBeams];
+    __shared__ int n_work_s;
+    __shared__ int stat_s[4];
+    extern __shared__ __align__(16) float q_s[];
+
+    const int lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5;
+    const int beam = w & 3;
+    const bool opens = w < kBeams;  // this warp has the open heap of its beam,
+    const bool results = !opens;    // the result heap
+    const int64_t b = blockIdx.x;
+    HeapEntry *open = open_s[beam], *res = res_s[beam];
+
+    for (int i = threadIdx.x; i < kBloomWords; i += kWideThreads) bloom[i] = 0;
+    for (int i = threadIdx.x; i < d; i += kWideThreads) q_s[i] = query[b * ldq + i];
+    for (int i = threadIdx.x; i < kBeams * (H + 2); i += kWideThreads) {
+        open_s[i / (H + 2)][i % (H + 2)] = HeapEntry{CUDART_INF_F, -1};
+        res_s[i / (H + 2)][i % (H + 2)] = HeapEntry{-CUDART_INF_F, -1};
+    }
+    if (threadIdx.x < 4) {
+        worst_s[threadIdx.x] = CUDART_INF_F;
+        stat_s[threadIdx.x] = 0;
+    }
+    PathBits<W> bits;  // of this warp's heap: larger children (open), smaller ones (result)
+    bits.clear();
+    float worst = CUDART_INF_F;  // result warps: the largest distance held
+    int n_expand = 0, n_eval = 0, n_rounds = 0;
+    const WalkLane WL = walk_lane(lane);
+    __syncthreads();
+
+    // What the two warps of a beam do with a list of up to 32 candidates, one per lane, in
+    // lane order: heap_replace / heap_pushpop of those below the limit of the moment.
+    auto fill_open = [&](float dist, int32_t value, bool valid) {
+        unsigned ahead = __ballot_sync(kAll, valid);
+        while (ahead != 0) {
+            const int leaf = bits.leaf(H);
+            const ReplaceLane r = bit_replace_load(open, H, leaf, lane);
+            const unsigned m = __ballot_sync(kAll, dist < r.limit) & ahead;
+            if (m == 0) break;
+            const int j = __ffs(m) - 1;
+            ahead &= 0xfffffffeu << j;
+            bit_replace_apply(open, leaf, r, __shfl_sync(kAll, dist, j),
+                              __shfl_sync(kAll, value, j), bits, lane);
+        }
+    };
+    auto fill_result = [&](float dist, int32_t id, bool valid) {  // returns: this lane's was taken
+        unsigned ahead = __ballot_sync(kAll, valid), taken = 0;
+        while (ahead != 0) {
+            const unsigned m = __ballot_sync(kAll, dist < worst) & ahead;
+            if (m == 0) break;
+            const int j = __ffs(m) - 1;
+            ahead &= 0xfffffffeu << j;
+            taken |= 1u << j;
+            bit_sink(res, H, HeapEntry{-__shfl_sync(kAll, dist, j), __shfl_sync(kAll, id, j)}, bits,
+                     lane);
+            worst = -res[1].k;
+        }
+        return ((taken >> lane) & 1u) != 0;
+    };
+
+    // ---- entries (traverse_cuda.cu:96-111): entry i belongs to beam i mod 4 ------
+    for (int base = 0; base < n_init; base += kSpare) {
+        const int n_here = min(kSpare, n_init - base);
+        if (threadIdx.x < n_here) {  // stage ids, rows, distances
+            const int64_t node = init_I[b * n_init + base + threadIdx.x];
+            int32_t row = -1;
+            if constexpr (Layout::kPacked) {
+                if (node >= 0 && node < L.n_nodes) row = __ldg(L.row_of + node);
+            }
+            slots[threadIdx.x] = make_int2(node < 0 ? -1 : static_cast<int32_t>(node), row);
+            cand_d[threadIdx.x] = init_D[b * n_init + base + threadIdx.x];
+        }
+        __syncthreads();
+        const int i = kBeams * lane + beam;  // this lane's entry
+        const bool have = i < n_here;
+        if (results) {  // admission test (:99) + result heap
+            const int32_t id = have ? slots[i].x : -1;
+            const float dist = have ? cand_d[i] : CUDART_INF_F;
+            // (a NaN passes the test but not the one of the result heap)
+            const bool admit = fill_result(dist, id, id >= 0) || (id >= 0 && dist != dist);
+            if (have && !admit) slots[i].x = -1;
+        }
+        __syncthreads();
+        if (opens) {
+            const int2 e = have ? slots[i] : make_int2(-1, -1);
+            const int32_t value = !Layout::kPacked ? e.x : e.y >= 0 ? e.y : -2;
+            fill_open(have ? cand_d[i] : CUDART_INF_F, value, e.x >= 0);
+        } else if (results) {  // bloom: the union of the admitted entries' bits
+            const int x = static_cast<int>(threadIdx.x) - kSpare;
+            const int32_t node = x < n_here ? slots[x].x : -1;
+            if (node >= 0) bloom_insert(bloom, node);
+        }
+        __syncthreads();
+    }
+    if (results && lane == 0) worst_s[beam] = worst;
+    __syncthreads();
+
+    // ---- rounds (traverse_cuda.cu:179-226) -----------------------------------------
+    int32_t ahead_v = -1;                      // open warps: the node whose row is on its way
+    int4 ahead_row = make_int4(-1, -1, 0, 0);  // (packed layout)
+    for (int step = 0; step < ef; ++step) {
+        ++n_rounds;
+        if (opens) {
+            // pop until there is a node with an adjacency row, or the beam gives up
+            // (:118-134); the heap is repaired while the row is on its way
+            const float bound = worst_s[beam];
+            int4 e = make_int4(-1, -1, 0, 0);
+            // every pop removes one element, so H + 1 pops always settle a beam
+            for (int guard = 0; guard <= H + 1; ++guard) {
+                const HeapEntry top = open[1];
+                const bool stop = top.v == -1 || top.k >= bound;
+                bool usable;
+                int4 got = make_int4(-1, -1, 0, 0);
+                if constexpr (Layout::kPacked) {
+                    usable = top.v >= 0;
+                    if (!stop && usable) {
+                        got = ahead_row;
+                        if (top.v != ahead_v)
+                            got = __ldg(L.nbr + static_cast<int64_t>(top.v) * n_nb + lane);
+                    }
+                } else {
+                    // ids come from the caller's entries and graph: one outside
+                    // [0, n_nodes) is treated as a node without an adjacency row
+                    usable = top.v >= 0 && top.v < L.n_nodes;
+                    if (!stop && usable) {
+                        const int64_t lo = __ldg(L.indptr + top.v), hi = __ldg(L.indptr + top.v + 1);
+                        usable = lo != hi;
+                        if (lane < min(hi - lo, static_cast<int64_t>(n_nb)))
+                            got.x = static_cast<int32_t>(__ldg(L.indices + lo + lane));
+                    }
+                }
+                bit_pop(open, H, bits, lane, WL);
+                if (stop) break;
+                if (!usable) continue;
+                if (Layout::kPacked && __shfl_sync(kAll, got.x, 0) == kEmptyRowTag) continue;
+                e = got;
+                ++n_expand;
+                break;
+            }
+            const int at = w * n_nb + lane;
+            row_s[at] = make_int2(e.x, e.y);
+            if constexpr (Layout::kPacked)
+                probe_s[at] = make_uint2(static_cast<uint32_t>(e.z), static_cast<uint32_t>(e.w));
+            else
+                probe_s[at] = probe_pack(bloom_prepare(e.x, lane));
+        }
+        __syncthreads();
+        if (w == 0) {
+            // bloom test-and-set in slot order, then compaction (:137-171): all loads, the
+            // 16 atomics back to back, the survivors in slot order
+            int2 ev[kBeams];
+            uint2 pv[kBeams];
+#pragma unroll
+            for (int bb = 0; bb < kBeams; ++bb) {
+                ev[bb] = row_s[bb * n_nb + lane];
+                pv[bb] = probe_s[bb * n_nb + lane];
+            }
+            uint32_t miss[kBeams];  // nonzero: some probed bit was clear before
+#pragma unroll
+            for (int bb = 0; bb < kBeams; ++bb) {
+                const BloomProbe pr = probe_unpack(pv[bb]);
+                miss[bb] = 0;
+#pragma unroll
+                for (int s = 0; s < kFnvSteps; ++s) {
+                    const uint32_t bit = ((pr.elected >> s) & 1u) << (pr.pos[s] & 31);
+                    miss[bb] |= ~atomicOr(&bloom[pr.pos[s] >> 5], bit) & bit;
+                    __syncwarp();
+                }
+            }
+            int off = 0;
+#pragma unroll
+            for (int bb = 0; bb < kBeams; ++bb) {
+                const unsigned m = __ballot_sync(kAll, miss[bb] != 0);
+                slots[miss[bb] != 0 ? off + __popc(m & ((1u << lane) - 1u)) : kSpare + lane] = ev[bb];
+                off += __popc(m);
+            }
+            n_work_s = off;  // warp-uniform
+        }
+        __syncthreads();
+        const int n_work = n_work_s;
+        if (n_work < kTeamsPerWarp) break;  // :182-184, uniform over the CTA
+        team_distances(L, slots, cand_d, kSpare, q_s, d, lane, w * kTeamsPerWarp + (lane >> 3),
+                       kWideThreads / kTeam, 0, n_work);
+        __syncthreads();
+        // heap inserts (:206-220): candidate j -> beam (j / 4) mod 4, ascending j; lane s
+        // holds position s of the beam's list
+        const int j = deal_index(lane, beam);  // in bounds
+        const bool have = lane < deal_count(n_work, beam);
+        const int2 e = slots[j];
+        const float dist = have ? cand_d[j] : CUDART_INF_F;
+        if (opens) {
+            if constexpr (Layout::kPacked) {
+                // (a heap holds strictly larger keys below a new root, an equal one stays
+                // behind it; distances are sums of squares: their bits order like them)
+                const unsigned key = __float_as_uint(dist);
+                const unsigned least = __reduce_min_sync(kAll, key);
+                const int first = __ffs(__ballot_sync(kAll, key == least)) - 1;
+                const int32_t best_v = __shfl_sync(kAll, e.y, first);
+                const HeapEntry top = open[1];
+                ahead_v = __uint_as_float(least) < top.k ? best_v : top.v;
+                if (ahead_v >= 0)
+                    ahead_row = __ldg(L.nbr + static_cast<int64_t>(ahead_v) * n_nb + lane);
+            }
+            fill_open(dist, !Layout::kPacked ? e.x : e.y, have);
+        } else if (results) {
+            fill_result(dist, e.x, have);
+            if (lane == 0) worst_s[beam] = worst;
+            if (stats != nullptr && w == kBeams) {
+                int valid = 0;
+                for (int jb = 0; jb < n_work; jb += 32)  // slots[jb + lane] is in bounds
+                    valid += (jb + lane < n_work) & (slots[jb + lane].y >= 0);
+                n_eval += __reduce_add_sync(kAll, valid);
+            }
+        }
+        beam_sync(beam);  // the worst result is visible to the open warp before it pops
+    }
+    __syncthreads();
+
+    // ---- store (:230-245): per beam worst -> best, into the open heaps' memory; sorted
+    // where no two keys among the entries that come out are equal, popped otherwise
+    const int n_discard = max(H - ef, 0), n_real = min(ef, H);
+    if (results) {
+        float k[H / 32];
+        int32_t v[H / 32];
+#pragma unroll
+        for (int x = 0; x < H / 32; ++x) {
+            const HeapEntry r = res[1 + lane * (H / 32) + x];
+            k[x] = r.k;
+            v[x] = r.v;
+        }
+        warp_sort(k, v, lane);
+        if (!warp_has_twins(k, v, n_discard, lane)) {
+#pragma unroll
+            for (int x = 0; x < H / 32; ++x) {
+                const int i = lane * (H / 32) + x - n_discard;
+                if (i >= 0) open[i] = HeapEntry{-k[x], v[x]};
+            }
+        } else {
+            for (int p = 0; p < n_discard + n_real; ++p) {
+                const HeapEntry r = res[1];
+                __syncwarp();
+                bit_sink(res, H, HeapEntry{CUDART_INF_F, -1}, bits, lane);
+                if (p >= n_discard && lane == 0) open[p - n_discard] = HeapEntry{-r.k, r.v};
+            }
+        }
+    }
+    __syncthreads();
+    {
+        int64_t *oI = out_I + b * kBeams * ef;
+        float *oD = out_D + b * kBeams * ef;
+        for (int i = threadIdx.x; i < kBeams * n_real; i += kWideThreads) {
+            const int bm = i / n_real, x = i - bm * n_real;
+            const HeapEntry r = open_s[bm][x];
+            oI[bm * ef + x] = r.v;
+            oD[bm * ef + x] = r.k;
+        }
+        // ef > H: the heap is exhausted, upstream keeps popping (-1, key +inf)
+        const int n_tail = ef - n_real;
+        for (int i = threadIdx.x; i < kBeams * n_tail; i += kWideThreads) {
+            const int bm = i / n_tail, x = n_real + (i - bm * n_tail);
+            oI[bm * ef + x] = -1;
+            oD[bm * ef + x] = -CUDART_INF_F;
+        }
+    }
+    if (stats != nullptr) {
+        int set = 0;
+        for (int i = threadIdx.x; i < kBloomWords; i += kWideThreads) set += __popc(bloom[i]);
+        set = __reduce_add_sync(kAll, set);
+        if (lane == 0) {
+            atomicAdd(&stat_s[3], set);
+            if (opens) atomicAdd(&stat_s[1], n_expand);
+            if (w == 0) stat_s[0] = n_rounds;
+            if (w == kBeams) stat_s[2] = n_eval;
+        }
+        __syncthreads();
+        if (threadIdx.x < 4) stats[b * 4 + threadIdx.x] = stat_s[threadIdx.x];
+    }
+}
+
 template <class Layout>
 static int launch(Layout L, int64_t *out_I, float *out_D, const float *query, int64_t ldq,
                   const int64_t *init_I, const float *init_D, int64_t batch, int d, int n_nb,
@@ -973,6 +1298,31 @@ static int launch(Layout L, int64_t *out_I, float *out_D, const float *query, in
     if (batch == 0) return PA_OK;
     dim3 grid(static_cast<unsigned>(batch)), block(kThreads);
     size_t dyn = sizeof(float) * d;
+    if (n_nb == 32) {
+        static int sm_count[64] = {};
+        int dev = 0, sms = 0;
+        PA_CUDA_TRY(cudaGetDevice(&dev));
+        if (dev >= 0 && dev < 64) {
+            if (sm_count[dev] == 0)
+                PA_CUDA_TRY(cudaDeviceGetAttribute(&sm_count[dev], cudaDevAttrMultiProcessorCount, dev));
+            sms = sm_count[dev];
+        }
+        if (batch <= static_cast<int64_t>(kWidePerSm) * sms) {
+#define PA_LAUNCH_WIDE(HS)                                                  \
+    traverse_wide_kernel<HS, Layout><<<grid, kWideThreads, dyn, stream>>>(  \
+        L, out_I, out_D, query, init_I, init_D, d, ldq, n_init, ef, stats)
+            switch (pa_heap_size_for(ef)) {
+                case 32: PA_LAUNCH_WIDE(32); break;
+                case 64: PA_LAUNCH_WIDE(64); break;
+                case 128: PA_LAUNCH_WIDE(128); break;
+                default: PA_LAUNCH_WIDE(256); break;
+            }
+#undef PA_LAUNCH_WIDE
+            count_launch();
+            PA_CUDA_TRY(cudaGetLastError());
+            return PA_OK;
+        }
+    }
 #define PA_LAUNCH(HS, CHS)                                                  \
     traverse_kernel<HS, CHS, Layout><<<grid, block, dyn, stream>>>(         \
         L, out_I, out_D, query, init_I, init_D, d, ldq, n_init, ef, stats)

@@ -187,3 +187,29 @@ def test_drop_in_call_switches_to_the_packed_form(oracle_lib):
     assert next(iter(extension._pack_cache.values()))["packed"] is None
     torch.cuda.synchronize()
     assert torch.equal(oI.cpu(), want[0])
+
+
+@pytest.mark.parametrize("grid", [None, 1.0, 4.0])
+@pytest.mark.parametrize("ef", [16, 33, 100, 128, 200, 256, 300])
+def test_few_and_many_queries_take_the_same_search(oracle_lib, ef, grid):
+    """Up to two queries per SM have eight warps each, more have four: same bits from
+    both, on vectors of a coarse grid, too, where equal distances leave the order of the
+    output to the layout of the heaps."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    p = dict(make_problem(n=4096, d=48, ratio=0.5, batch=40, n_init=160, seed=9))
+    if grid is not None:
+        p["storage"] = (torch.round(p["storage"] * grid) / grid).contiguous()
+        p["query"] = (torch.round(p["query"] * grid) / grid).contiguous()
+        full = torch.round(p["full"] * grid) / grid
+        diff = p["query"].unsqueeze(1) - full[p["initial_I"]]
+        p["initial_D"] = (diff * diff).sum(-1).contiguous()
+    want = run_oracle(oracle_lib, p, ef)
+    if grid == 1.0:
+        kept = want[1][0, 0][want[0][0, 0] >= 0]
+        assert kept.unique().numel() < kept.numel()
+    many = (2 * sms) // 40 + 1
+    tiled = dict(p, **{k: p[k].repeat(many, 1) for k in ("query", "initial_I", "initial_D")})
+    for layout in ("csr", "packed"):
+        assert_same(run_gpu(p, ef, layout), want)
+        got = run_gpu(tiled, ef, layout)
+        assert_same(got, [x.repeat(many, *[1] * (x.dim() - 1)) for x in want])
