@@ -222,3 +222,24 @@ def test_ragged_chunks_and_empty_submit(small_index):
     assert out[0].shape == (0, k)
     with pytest.raises(RuntimeError):                                  # k beyond the row
         stage.search_host(q, ef, k=4 * ef + 1)
+
+
+def test_chunks_beyond_one_wave(small_index):
+    """Chunks are taken together up to a wave of queries; a batch of several waves is still
+    cut, its pieces alternating over the streams: rows as from one launch, in every mode."""
+    index, x, q, w = small_index
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B, ef, k = 2 * 7 * sms + 77, 20, 6
+    many = q.repeat(B // q.size(0) + 1, 1)[:B].contiguous()
+    try:
+        index.to("cuda", max_batch=B, max_ef=32)
+        stage = index.stage
+        for mode in ({}, {"stage2": True}, {"k": k}):
+            rot = torch.empty(B, q.size(1))
+            want_I, want_D, _ = stage.search_host(many, ef, **mode)
+            got_I, got_D, _ = stage.search_host(many, ef, chunk=100, rotated=rot, **mode)
+            assert torch.equal(want_I, got_I) and torch.equal(want_D, got_D)
+            assert torch.equal(got_I[:q.size(0)], got_I[q.size(0):2 * q.size(0)])
+        assert torch.equal(rot[:q.size(0)], rot[q.size(0):2 * q.size(0)])
+    finally:
+        index.to("cuda", max_batch=256, max_ef=128)
