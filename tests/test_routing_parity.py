@@ -96,3 +96,21 @@ def test_projection_matches_oracle(oracle_lib, B, d, d_out):
     dg = torch.cdist(got.double(), x.double()).square()
     dw = torch.cdist(want.double(), x.double()).square()
     assert ((dg - dw).abs() / dw).max().item() <= RTOL
+
+
+@pytest.mark.parametrize("n_r,n_l,d,B", [(2, 32, 4, 3), (33, 96, 100, 255), (7, 32, 132, 256),
+                                         (64, 64, 1540, 41), (300, 32, 36, 9)])
+def test_routing_of_small_batches(oracle_lib, n_r, n_l, d, B):
+    """Up to 256 queries the router scores come from the kernel for a few rows: odd router
+    counts, dimensions beyond one slice of it, leaves in several passes."""
+    from pilotann_b200 import extension
+    x, rv, en, ev = _tables(20000, d, n_r, n_l, seed=n_r + d)
+    g = torch.Generator().manual_seed(B)
+    q = 2.0 * (torch.rand(B, d, generator=g) - 0.5)
+    router, dist, ids = extension.routing_cuda(q.cuda(), rv.cuda(), en.cuda(), ev.cuda(),
+                                               with_ids=True)
+    w_router, w_dist, w_ids = oracle_lib.route(q, rv, en, ev)
+    assert torch.equal(router.cpu(), w_router) and torch.equal(ids.cpu(), w_ids)
+    assert torch.allclose(dist.cpu(), w_dist, rtol=RTOL, atol=0.0)
+    alone = extension.routing_cuda(q[-1:].cuda(), rv.cuda(), en.cuda(), ev.cuda())
+    assert torch.equal(alone[1][0], dist[-1])
