@@ -27,11 +27,14 @@
 // A heap operation is executed by a group of 8 lanes, one lane per level of the
 // root-to-leaf path, the four beams side by side in one warp.  The path is not
 // found by walking keys in shared memory: each heap keeps, in registers, one bit
-// per internal node for "right child smaller" and (open heaps) one for "right
-// child larger"; following them is a few integer instructions, after which every
-// lane derives its own node of the path by a shift (1-based heap indices).  The
-// bits of the nodes whose children changed are refreshed with an 8-lane OR per
-// word.  The element layout of the heaps is exactly upstream's after every
+// per internal node -- "right child smaller" in the result heaps, "right child
+// larger" in the open heaps; following them is a few integer instructions, after
+// which every lane derives its own node of the path by a shift (1-based heap
+// indices).  The bits of the nodes whose children changed are refreshed with an
+// 8-lane OR for the top five levels and a shuffle for each deeper one.  (With both
+// kinds of bits in the open heaps and an OR per word the kernel took, us: 1024 queries
+// at ef 128, 192 and 256 1136, 1894 and 408, now 1094, 1721 and 375; 16384 queries at
+// ef 256 4182, now 3615.)  The element layout of the heaps is exactly upstream's after every
 // operation (heapq.cuh:13-87), which is what makes evictions -- and therefore
 // results -- identical.
 //
@@ -134,23 +137,29 @@ __device__ __forceinline__ uint32_t group_or(uint32_t mine) {
     return mine;
 }
 
-// XOR `mine` (a single bit, or 0) into the word that holds node n, combined
-// over the 8 lanes of a group.
-template <int W>
-__device__ __forceinline__ void flip_bits(uint32_t (&w)[W], uint32_t mine, unsigned n) {
-    if constexpr (W == 1) {
-        w[0] ^= group_or(mine);
-    } else {
-#pragma unroll
-        for (int i = 0; i < W; ++i)
-            w[i] ^= group_or((n >> 5) == static_cast<unsigned>(i) ? mine : 0u);
-    }
-}
-
 struct GroupCtx {
     unsigned g;      // lane within the group = level handled
     unsigned gshift; // first lane of this group
 };
+
+// XOR `mine` (a single bit, or 0) into the word that holds node n, combined over the 8
+// lanes of a group.  Lane t of a group speaks for a node of level t: levels 0-4 are the
+// five bits of word 0 that need an OR, word 1 has the word of lane 5 alone, words 2 and 3
+// that of lane 6.
+template <int W>
+__device__ __forceinline__ void flip_bits(uint32_t (&w)[W], uint32_t mine, unsigned n,
+                                          const GroupCtx &c) {
+    if constexpr (W == 1) {
+        w[0] ^= group_or(mine);
+    } else {
+        w[0] ^= group_or(c.g < 5 ? mine : 0u);
+        w[1] ^= __shfl_sync(kFull, mine, 5, kGroup);
+        if constexpr (W == 4) {
+            w[2] ^= __shfl_sync(kFull, (n & 32u) ? 0u : mine, 6, kGroup);
+            w[3] ^= __shfl_sync(kFull, (n & 32u) ? mine : 0u, 6, kGroup);
+        }
+    }
+}
 
 // ---- heap operations, one group of 8 lanes per heap --------------------------
 // K / V: the heap's arrays in shared memory (0-based storage of 1-based nodes),
@@ -171,11 +180,10 @@ template <typename V> struct SinkPath {
     V av;
 };
 
-template <int H, int W, typename V>
-__device__ __forceinline__ SinkPath<V> sink_load(const float *K, const V *Vv,
-                                                 const uint32_t (&sb)[W], const GroupCtx &c) {
+template <int H, typename V>
+__device__ __forceinline__ SinkPath<V> sink_load_at(const float *K, const V *Vv,
+                                                    const GroupCtx &c, unsigned leaf) {
     SinkPath<V> p;
-    const unsigned leaf = follow_bits<H, W>(sb);
     const unsigned L = 31u - __clz(leaf);
     const unsigned t = c.g + 1u;  // this lane's level on the path
     p.in = t <= L;
@@ -187,10 +195,16 @@ __device__ __forceinline__ SinkPath<V> sink_load(const float *K, const V *Vv,
     return p;
 }
 
-template <int H, int W, bool kHasLb, typename V>
-__device__ __forceinline__ float sink_apply(float *K, V *Vv, uint32_t (&sb)[W], uint32_t (&lb)[W],
-                                            const GroupCtx &c, const SinkPath<V> &p, bool active,
-                                            float k, V v) {
+template <int H, int W, typename V>
+__device__ __forceinline__ SinkPath<V> sink_load(const float *K, const V *Vv,
+                                                 const uint32_t (&sb)[W], const GroupCtx &c) {
+    return sink_load_at<H, V>(K, Vv, c, follow_bits<H, W>(sb));
+}
+
+// kLarger: `bits` are those of the larger children (open heap), else of the smaller ones.
+template <int H, int W, bool kLarger, typename V>
+__device__ __forceinline__ float sink_apply(float *K, V *Vv, uint32_t (&bits)[W], const GroupCtx &c,
+                                            const SinkPath<V> &p, bool active, float k, V v) {
     const unsigned t = c.g + 1u;  // this lane's level on the path
     const unsigned node = p.node;
     const bool on = active && p.in;
@@ -217,21 +231,45 @@ __device__ __forceinline__ float sink_apply(float *K, V *Vv, uint32_t (&sb)[W], 
     const float left = odd ? p.sk : nk, right = odd ? nk : p.sk;
     const unsigned parent = node >> 1;
     const bool upd = moves && sib_ok;
-    const uint32_t s_flip = (right < left) != (bit_at<W>(sb, parent) != 0);
-    flip_bits<W>(sb, (upd && s_flip) ? (1u << (parent & 31u)) : 0u, parent);
-    if constexpr (kHasLb) {
-        const uint32_t l_flip = (right > left) != (bit_at<W>(lb, parent) != 0);
-        flip_bits<W>(lb, (upd && l_flip) ? (1u << (parent & 31u)) : 0u, parent);
-    }
+    const bool flip = (kLarger ? right > left : right < left) != (bit_at<W>(bits, parent) != 0);
+    flip_bits<W>(bits, (upd && flip) ? (1u << (parent & 31u)) : 0u, parent, c);
     __syncwarp();
     return cnt == 0 ? k : a_first;
 }
 
-template <int H, int W, bool kHasLb, typename V>
-__device__ __forceinline__ float group_sink(float *K, V *Vv, uint32_t (&sb)[W], uint32_t (&lb)[W],
-                                            const GroupCtx &c, bool active, float k, V v) {
+template <int H, int W, typename V>
+__device__ __forceinline__ float group_sink(float *K, V *Vv, uint32_t (&sb)[W], const GroupCtx &c,
+                                            bool active, float k, V v) {
     const SinkPath<V> p = sink_load<H, W, V>(K, Vv, sb, c);
-    return sink_apply<H, W, kHasLb, V>(K, Vv, sb, lb, c, p, active, k, v);
+    return sink_apply<H, W, false, V>(K, Vv, sb, c, p, active, k, v);
+}
+
+// heap_pop of the open heap, whose bits are those of its larger children: the leaf at the
+// end of the smaller children is found from the keys, three levels a step (lane g of a
+// group looks at the g-th node of the seven).  One pop a round runs under the fetch of the
+// neighbour rows; the bits for it would be refreshed in each of the round's inserts.
+template <int H, int W, typename V>
+__device__ __forceinline__ void group_pop(float *K, V *Vv, uint32_t (&lb)[W], const GroupCtx &c,
+                                          bool active, V none) {
+    constexpr int kDecisions = HeapShape<H>::kLog - 1;  // nodes below H/2 have two children
+    const unsigned depth = c.g == 0 || c.g == 7 ? 0u : c.g < 3 ? 1u : 2u;
+    const unsigned off = c.g == 7 ? 0u : c.g + 1u - (1u << depth);
+    unsigned a = 1;
+#pragma unroll
+    for (int l = 0; l < kDecisions; l += 3) {
+        const int levels = kDecisions - l < 3 ? kDecisions - l : 3;
+        const unsigned node = (a << depth) + off;
+        const unsigned at = node < H / 2 ? node : 1u;
+        const bool right = K[2 * at] < K[2 * at - 1];
+        const unsigned B = __ballot_sync(kFull, right) >> c.gshift;
+        unsigned n = 1;
+#pragma unroll
+        for (int t = 0; t < levels; ++t) n = (n << 1) | ((B >> (n - 1u)) & 1u);
+        a = (a << levels) + n - (1u << levels);
+    }
+    const unsigned leaf = a == H / 2 ? static_cast<unsigned>(H) : a;
+    const SinkPath<V> p = sink_load_at<H, V>(K, Vv, c, leaf);
+    sink_apply<H, W, true, V>(K, Vv, lb, c, p, active, CUDART_INF_F, none);
 }
 
 // upstream heap_replace (heapq.cuh:47-77): walk to a leaf along the larger
@@ -263,8 +301,8 @@ __device__ __forceinline__ ReplacePath<V> replace_load(const float *K, const V *
 }
 
 template <int H, int W, typename V>
-__device__ __forceinline__ void replace_apply(float *K, V *Vv, uint32_t (&sb)[W],
-                                              uint32_t (&lb)[W], const GroupCtx &c, unsigned leaf,
+__device__ __forceinline__ void replace_apply(float *K, V *Vv, uint32_t (&lb)[W],
+                                              const GroupCtx &c, unsigned leaf,
                                               const ReplacePath<V> &p, bool accept, float k, V v) {
     const unsigned L = p.L;
     const unsigned t = c.g;  // ancestors: levels 0 .. L-1
@@ -289,29 +327,27 @@ __device__ __forceinline__ void replace_apply(float *K, V *Vv, uint32_t (&sb)[W]
     const bool odd = child & 1u;
     const float left = odd ? p.sk : nk, right = odd ? nk : p.sk;
     const bool upd = on && t + 1u >= s && has_sib;
-    const bool s_flip = (right < left) != (bit_at<W>(sb, node) != 0);
-    const bool l_flip = (right > left) != (bit_at<W>(lb, node) != 0);
-    flip_bits<W>(sb, (upd && s_flip) ? (1u << (node & 31u)) : 0u, node);
-    flip_bits<W>(lb, (upd && l_flip) ? (1u << (node & 31u)) : 0u, node);
+    // the path went to this child: right if strictly larger than its sibling
+    const bool flip = odd ? !(right > left) : right > left;
+    flip_bits<W>(lb, (upd && flip) ? (1u << (node & 31u)) : 0u, node, c);
     __syncwarp();
 }
 
 template <int H, int W, typename V>
-__device__ __forceinline__ void group_replace_at(float *K, V *Vv, uint32_t (&sb)[W],
-                                                 uint32_t (&lb)[W], const GroupCtx &c,
-                                                 unsigned leaf, bool accept, float k, V v) {
+__device__ __forceinline__ void group_replace_at(float *K, V *Vv, uint32_t (&lb)[W],
+                                                 const GroupCtx &c, unsigned leaf, bool accept,
+                                                 float k, V v) {
     const ReplacePath<V> p = replace_load<H, V>(K, Vv, c, leaf);
-    replace_apply<H, W, V>(K, Vv, sb, lb, c, leaf, p, accept, k, v);
+    replace_apply<H, W, V>(K, Vv, lb, c, leaf, p, accept, k, v);
 }
 
 template <int H, int W, typename V>
-__device__ __forceinline__ void group_replace(float *K, V *Vv, uint32_t (&sb)[W],
-                                              uint32_t (&lb)[W], const GroupCtx &c, bool active,
-                                              float k, V v) {
+__device__ __forceinline__ void group_replace(float *K, V *Vv, uint32_t (&lb)[W],
+                                              const GroupCtx &c, bool active, float k, V v) {
     const unsigned leaf = follow_bits<H, W>(lb);
     const bool accept = active && k < K[leaf - 1];
     if (!__any_sync(kFull, accept)) return;
-    group_replace_at<H, W>(K, Vv, sb, lb, c, leaf, accept, k, v);
+    group_replace_at<H, W>(K, Vv, lb, c, leaf, accept, k, v);
 }
 
 // ---- distance (upstream traverse_cuda.cu:18-43) -------------------------------
@@ -532,9 +568,9 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
     int2 *oval = open_val[beam];
     float *rkey = res_key[beam];
     int32_t *rid = res_id[beam];
-    uint32_t o_sb[W], o_lb[W], r_sb[W];  // all keys equal at start: all bits 0
+    uint32_t o_lb[W], r_sb[W];  // all keys equal at start: all bits 0
 #pragma unroll
-    for (int i = 0; i < W; ++i) o_sb[i] = o_lb[i] = r_sb[i] = 0;
+    for (int i = 0; i < W; ++i) o_lb[i] = r_sb[i] = 0;
     float r_root = -CUDART_INF_F;  // warp 1: root key of the result heap
     int n_expand = 0, n_eval = 0, n_rounds = 0;
 
@@ -563,7 +599,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                 if (have && !admit && gc.g == 0) slots[i].x = -1;
                 const bool push = admit && (-dist > r_root);
                 if (__any_sync(kFull, push)) {
-                    const float root = group_sink<H, W, false>(rkey, rid, r_sb, r_sb, gc, push,
+                    const float root = group_sink<H, W>(rkey, rid, r_sb, gc, push,
                                                                -dist, e.x);
                     if (push) r_root = root;
                 }
@@ -576,7 +612,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                 const bool have = i < n_here;
                 const int2 e = have ? slots[i] : make_int2(-1, -1);
                 const float dist = have ? cand_d[i] : 0.0f;
-                group_replace<H, W>(okey, oval, o_sb, o_lb, gc, have && e.x >= 0, dist, e);
+                group_replace<H, W>(okey, oval, o_lb, gc, have && e.x >= 0, dist, e);
             }
         } else if (w >= 2) {  // bloom: the union of the admitted entries' bits
             for (int i = 32 * (w - 2) + lane; i < n_here; i += kThreads - 64) {
@@ -632,8 +668,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                     // case: the popped nodes are published first and the heaps are
                     // repaired while the neighbour rows are on their way.
                     if (__any_sync(kFull, pending && !settle))
-                        group_sink<H, W, true>(okey, oval, o_sb, o_lb, gc, pending, CUDART_INF_F,
-                                               make_int2(-1, -1));
+                        group_pop<H, W>(okey, oval, o_lb, gc, pending, make_int2(-1, -1));
                     else
                         deferred = pending;
                     u_node = settle ? (stop ? -1 : top_v.x) : u_node;
@@ -669,8 +704,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                         : make_int4(-1, -1, 0, 0);
                 // the open warp repairs its heaps while its row is on its way
                 if (w == 0 && __any_sync(kFull, deferred)) {
-                    group_sink<H, W, true>(okey, oval, o_sb, o_lb, gc, deferred, CUDART_INF_F,
-                                           make_int2(-1, -1));
+                    group_pop<H, W>(okey, oval, o_lb, gc, deferred, make_int2(-1, -1));
                     deferred = false;
                 }
                 if (fetch_w) {
@@ -689,8 +723,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                 }
             } else {
                 if (w == 0 && __any_sync(kFull, deferred)) {
-                    group_sink<H, W, true>(okey, oval, o_sb, o_lb, gc, deferred, CUDART_INF_F,
-                                           make_int2(-1, -1));
+                    group_pop<H, W>(okey, oval, o_lb, gc, deferred, make_int2(-1, -1));
                     deferred = false;
                 }
                 if (fetch_w) {
@@ -822,7 +855,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                             if (!__any_sync(kFull, found)) break;
                             const unsigned pos = found ? __ffs(m) - 1 : 0u;
                             const float key = list_at(cd, pos);
-                            replace_apply<H, W>(okey, oval, o_sb, o_lb, gc, leaf, path, found, key,
+                            replace_apply<H, W>(okey, oval, o_lb, gc, leaf, path, found, key,
                                                 slots[deal_index(pos, beam)]);
                             if (found) ahead = 0xfffffffeu << pos;
                             leaf = follow_bits<H, W>(o_lb);
@@ -850,7 +883,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                         const unsigned pos = found ? __ffs(m) - 1 : 0u;
                         const float key = list_at(cd, pos);
                         const float root = sink_apply<H, W, false>(
-                            rkey, rid, r_sb, r_sb, gc, path, found, -key,
+                            rkey, rid, r_sb, gc, path, found, -key,
                             slots[deal_index(pos, beam)].x);
                         if (found) { r_root = root; ahead = 0xfffffffeu << pos; }
                     }
@@ -873,7 +906,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                         const bool found = s < count;
                         if (!__any_sync(kFull, found)) break;
                         const int j = found ? deal_index(s, beam) : 0;
-                        group_replace_at<H, W>(okey, oval, o_sb, o_lb, gc, leaf, found, cand_d[j],
+                        group_replace_at<H, W>(okey, oval, o_lb, gc, leaf, found, cand_d[j],
                                                slots[j]);
                         s += found;
                         leaf = follow_bits<H, W>(o_lb);
@@ -885,7 +918,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
                         const bool found = s < count;
                         if (!__any_sync(kFull, found)) break;
                         const int j = found ? deal_index(s, beam) : 0;
-                        const float root = group_sink<H, W, false>(rkey, rid, r_sb, r_sb, gc, found,
+                        const float root = group_sink<H, W>(rkey, rid, r_sb, gc, found,
                                                                    -cand_d[j], slots[j].x);
                         if (found) { r_root = root; ++s; }
                     }
@@ -928,7 +961,7 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
         for (int p = 0; p < n_discard + n_real; ++p) {
             const float key = rkey[0];
             const int32_t id = rid[0];
-            group_sink<H, W, false>(rkey, rid, r_sb, r_sb, gc, true, CUDART_INF_F, int32_t(-1));
+            group_sink<H, W>(rkey, rid, r_sb, gc, true, CUDART_INF_F, int32_t(-1));
             const int i = p - n_discard;
             oval[(i >= 0 && gc.g == 0) ? i : H + static_cast<int>(gc.g)] =
                 make_int2(id, __float_as_int(-key));
