@@ -413,6 +413,69 @@ def test_result_list_of_every_capacity(oracle_lib, ef, k, spoil):
         assert torch.equal(st.cpu(), w_st), top
 
 
+@pytest.mark.parametrize("per_sm,d,ef", [(2, 48, 24), (2, 768, 40), (4, 768, 128), (4, 48, 256),
+                                         (2, 2048, 64)])
+def test_ctas_for_few_queries_per_sm(oracle_lib, per_sm, d, ef):
+    """Two and four queries per SM: CTAs of 16 and 8 warps, with long rows and short ones.
+    Bit for bit the oracle's."""
+    from pilotann_b200 import extension
+    from helpers import make_problem
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    base, n, d_p, k = 24, 6000, 16, 10
+    g = torch.Generator().manual_seed(d + ef)
+    p = make_problem(n=n, d=d, ratio=0.5, batch=base, n_init=32, seed=800, exact_entries=False)
+    full, q = p["full"], p["query"]
+    ids = p["nodelist"][torch.randint(p["nodelist"].numel(), (base, 4 * ef), generator=g)]
+    dist = ((q[:, :d_p].unsqueeze(1) - full[ids][:, :, :d_p]) ** 2).sum(-1).contiguous()
+    nbr, row_of = extension.pack_graph(p["indptr"].cuda(), p["indices"].cuda(), p["mapping"].cuda(),
+                                       p["storage"].size(0), 32)
+    full_nbr = extension.pack_fullgraph(p["full_indptr"].cuda(), p["full_indices"].cuda(), 32)
+    w_I, w_D, w_st = oracle_lib.refine_ex(ids.clone(), dist.clone(), [p["indptr"], p["indices"]],
+                                          [p["full_indptr"], p["full_indices"]], full, q, k, ef,
+                                          d_p, gpu_order=True, with_stats=True)
+    times = per_sm * sms // base
+    B = times * base
+    pool = extension.VisitedPool(n, B)
+    st = torch.zeros(B, 4, dtype=torch.int32, device="cuda")
+    for _ in range(2):                                     # the second launch finds used slots
+        t_I, t_D = extension.refine(ids.repeat(times, 1).cuda(), dist.repeat(times, 1).cuda(),
+                                    q.repeat(times, 1).cuda(), full.cuda(), nbr, row_of, full_nbr,
+                                    pool, ef, d_p, k=k, stats=st)
+        torch.cuda.synchronize()
+        assert torch.equal(t_I.cpu(), w_I.repeat(times, 1))
+        assert torch.equal(t_D.cpu().view(torch.int32), w_D.view(torch.int32).repeat(times, 1))
+        assert torch.equal(st.cpu(), w_st.repeat(times, 1))
+
+
+@pytest.mark.parametrize("d,d_p", [(36, 4), (36, 12), (36, 32), (68, 4), (100, 36), (104, 36)])
+def test_short_residuals(oracle_lib, d, d_p):
+    """Seeds completed over at most 32 and 64 trailing dimensions share a warp by four and
+    by two; one more group of four dimensions takes the whole warp."""
+    from pilotann_b200 import extension
+    from helpers import make_problem
+    B, n, ef = 16, 3000, 37
+    g = torch.Generator().manual_seed(d * 100 + d_p)
+    p = make_problem(n=n, d=d, ratio=0.5, batch=B, n_init=32, seed=900 + d)
+    full, q = p["full"], p["query"]
+    ids = p["nodelist"][torch.randint(p["nodelist"].numel(), (B, 4 * ef), generator=g)]
+    ids[torch.rand(B, 4 * ef, generator=g) < 0.2] = -1
+    dist = ((q[:, :d_p].unsqueeze(1) - full[ids.clamp_min(0)][:, :, :d_p]) ** 2).sum(-1)
+    dist[ids < 0] = float("inf")
+    dist = dist.contiguous()
+    nbr, row_of = extension.pack_graph(p["indptr"].cuda(), p["indices"].cuda(), p["mapping"].cuda(),
+                                       p["storage"].size(0), 32)
+    pool = extension.VisitedPool(n, B)
+    t_I, t_D = extension.refine(ids.cuda(), dist.cuda(), q.cuda(), full.cuda(), nbr, row_of, None,
+                                pool, ef, d_p)
+    torch.cuda.synchronize()
+    w_I, w_D = ids.clone(), dist.clone()
+    oracle_lib.refine_ex(w_I, w_D, [p["indptr"], p["indices"]],
+                         [p["full_indptr"], p["full_indices"]], full, q, 10, ef, d_p,
+                         gpu_order=True, stages=2)
+    assert torch.equal(t_I.cpu(), w_I)
+    assert torch.equal(t_D.cpu().view(torch.int32), w_D.view(torch.int32))
+
+
 def test_replay_of_upstream_fixtures():
     """Outputs of upstream ``traverse_refine`` recorded by tests/golden/make_golden.py
     (CPU, no GPU involved), replayed through the refinement kernel without the
