@@ -13,7 +13,7 @@
 //
 // The candidates are consumed where the traversal left them, in HBM; nothing of
 // the handoff crosses PCIe.  One CTA of five warps (three for rows of at most 512
-// bytes) per query, persistent: CTA i owns slot i of the visited-set pool
+// bytes; sixteen or eight while the SMs have few queries) per query, persistent: CTA i owns slot i of the visited-set pool
 // (visited.cu), starts on query i and claims further queries from a counter.
 // Warp 0 is the heap warp, the other warps gather: adjacency row, visited marks,
 // vector rows, distances.  Four serial pieces of upstream's routine -- the result
@@ -54,8 +54,8 @@
 
 namespace pa {
 
-// Warp 0 runs the heaps, the other warps gather.  The kernel is compiled for CTAs of
-// up to five warps; vector rows of at most 512 bytes are served by two gather warps
+// Warp 0 runs the heaps, the other warps gather.  Where the SMs are full the kernel has
+// up to five warps (wider CTAs: refine_launch_for); vector rows of at most 512 bytes are served by two gather warps
 // (96 threads), which lets twelve instead of seven queries share an SM -- at those
 // sizes the heap warp, not the gather, sets the pace of a query -- or by three when
 // the batch leaves room for them (nine queries per SM).
@@ -68,7 +68,7 @@ namespace pa {
 #ifndef PA_REFINE_NARROW_DIM
 #define PA_REFINE_NARROW_DIM 128
 #endif
-constexpr int kRefThreads = 160;  // what the kernel is compiled for
+constexpr int kRefThreads = 160;  // what that kernel is compiled for
 constexpr int kRefThreadsWide = PA_REFINE_WIDE_THREADS;
 constexpr int kRefThreadsNarrow = PA_REFINE_NARROW_THREADS;
 constexpr int kNarrowMaxDim = PA_REFINE_NARROW_DIM;
