@@ -13,8 +13,9 @@
 //
 // The candidates are consumed where the traversal left them, in HBM; nothing of
 // the handoff crosses PCIe.  One CTA of five warps (three for rows of at most 512
-// bytes; sixteen or eight while the SMs have few queries) per query, persistent: CTA i owns slot i of the visited-set pool
-// (visited.cu), starts on query i and claims further queries from a counter.
+// bytes; sixteen or eight while the SMs have few queries) per query, persistent:
+// CTA i owns slot i of the visited-set pool (visited.cu), starts on query i and
+// claims further queries from a counter.
 // Warp 0 is the heap warp, the other warps gather: adjacency row, visited marks,
 // vector rows, distances.  Four serial pieces of upstream's routine -- the result
 // heap, pushing the seeds into the open heap of the two-expansion stage, seeding the
@@ -763,6 +764,7 @@ __device__ __forceinline__ bool brief_prepare(const RefShared &S, int n_seed, Re
         if (S.c_id[i] < 0) continue;
         const float dist = S.c_d[i];
         if (!(dist >= 0.0f && dist < CUDART_INF_F)) bad = true;
+        if (dist != dist) ctl->rerun = 1;  // NaN in the open heap: see search_stage
         atomicMin(&ctl->m1, (static_cast<unsigned long long>(__float_as_uint(dist)) << 32) | i);
     }
     if (bad) ctl->tie = 1;
@@ -1066,8 +1068,8 @@ __device__ __noinline__ void upstream_output(const RefineArgs &A, const RefCtl *
 // are that stage's output.  n_check: how many leading entries of the output have to be
 // upstream's in the order of equal distances, too.  Returns expansions and
 // evaluations through ctl->st, and false (CTA-uniform) if the query
-// has to be run on the array heaps (R > 0 only: a NaN distance, which upstream's tests
-// let into the heaps, or equal distances after more admissions than the log holds).
+// has to be run on the array heaps (R > 0 only: a NaN distance, of a neighbour or of a
+// seed, which upstream's tests let into the heaps, or equal distances after more admissions than the log holds).
 template <int R>
 __device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShared &S,
                                              const RefGraph &G, uint8_t *vis, uint8_t marker,
