@@ -230,7 +230,8 @@ int pa_stage_search(pa_stage *stage, const float *host_query, float *host_rotate
                     int ef_search, int64_t chunk);
 
 /* Device-resident variant (inputs already in HBM, outputs stay there);
- * asynchronous on the stage's first stream; dev_query is the raw query.
+ * asynchronous on the stage's first stream; dev_query is the raw query (16-byte
+ * aligned when index.VT == NULL, as every vector of the index has to be).
  * dev_stats may be NULL. Returns after enqueueing. */
 int pa_stage_search_device(pa_stage *stage, const float *dev_query,
                            int64_t *dev_out_I, float *dev_out_D, int64_t batch,

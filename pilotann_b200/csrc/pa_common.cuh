@@ -47,6 +47,8 @@ int router_norms_launch(float *rnorm2, const float *route_vectors, int n_routers
                         cudaStream_t stream);
 int gemm_tf32x3_launch(float *out, const float *A, const float *B, int M, int N, int K,
                        int64_t lda, int64_t ldb, int64_t ldo, cudaStream_t stream);
+// rows of A and B can be read as aligned float4 (a tensor map wants the same)
+bool gemm_operands_ok(const float *A, const float *B, int K, int64_t lda, int64_t ldb);
 int gemm_small_launch(float *out, const float *A, const float *B, int M, int N, int K, int64_t lda,
                       int64_t ldb, int64_t ldo, cudaStream_t stream);
 const int *gemm_status_address();

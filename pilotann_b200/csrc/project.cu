@@ -61,7 +61,8 @@ project_kernel(float *__restrict__ out, const float *__restrict__ query,
 // shared memory; fp32 fma, 24 terms per lane and slice, butterfly over the lanes.  64
 // columns, K = 128: 1 row 5.2 -> 1.9 us, 256 rows 6.9 -> 4.1.  (Not for the rotation of the
 // queries: its results differ from the tensor cores' by 6e-6 at K = 768, fifty times
-// what they are off themselves, and a search decides by its input's last bits.)
+// what they are off themselves, and a search decides by its input's last bits.)  Reads
+// aligned float4 rows: callers see to gemm_operands_ok.
 constexpr int kSmallRows = 8;        // rows of A per CTA
 constexpr int kSmallWarps = 4;
 constexpr int kSmallSlice = 768;     // floats of K per pass: six float4 a lane
@@ -342,7 +343,7 @@ __global__ void bounded_wait_selftest_kernel(uint32_t polls) {
     }
 }
 
-static bool gemm_operands_ok(const float *A, const float *B, int K, int64_t lda, int64_t ldb) {
+bool gemm_operands_ok(const float *A, const float *B, int K, int64_t lda, int64_t ldb) {
     return K % 4 == 0 && lda % 4 == 0 && ldb % 4 == 0 && aligned16(A) && aligned16(B);
 }
 

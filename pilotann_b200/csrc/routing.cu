@@ -200,8 +200,9 @@ int route_launch(int64_t *router, float *leaf_D, int64_t *leaf_I, const float *q
     if (batch == 0) return PA_OK;
     const bool tensor = dots_ws != nullptr && rnorm2 != nullptr && route_vectors != nullptr &&
                         n_routers > 1 && d % 4 == 0 && ldq % 4 == 0;
-    // up to 256 queries by gemm_small_kernel (the scores only shortlist)
-    const bool small = tensor && batch <= 256;
+    // up to 256 queries by gemm_small_kernel (the scores only shortlist); operands it
+    // cannot read go to the other one, whose tensor map refuses them
+    const bool small = tensor && batch <= 256 && gemm_operands_ok(query, route_vectors, d, ldq, d);
     if (tensor) {
         const auto scores = small ? gemm_small_launch : gemm_tf32x3_launch;
         int rc = scores(dots_ws, query, route_vectors, static_cast<int>(batch), n_routers, d, ldq,

@@ -108,6 +108,19 @@ static int check_mode(pa_stage *st, int mode, int ef, int k) {
     return PA_OK;
 }
 
+// The kernels read vectors as float4.  Asked for before anything is enqueued; queries
+// that are rotated first may lie anywhere (project_launch has a kernel for those).
+static int check_alignment(const pa_stage *st, int mode, const float *searched_query) {
+    const pa_stage_index &ix = st->ix;
+    PA_REQUIRE(aligned16(ix.storage) && aligned16(ix.packed_nbr) && aligned16(ix.entry_vectors) &&
+                   aligned16(ix.route_vectors),
+               "the stage's packed graph, storage, entry and route vectors must be 16-byte aligned");
+    PA_REQUIRE(mode == PA_OUT_HANDOFF || aligned16(st->rx.storage_full),
+               "the stage's full-dimension vectors must be 16-byte aligned");
+    PA_REQUIRE(aligned16(searched_query), "queries must be 16-byte aligned (the stage has no rotation)");
+    return PA_OK;
+}
+
 // Row length of a mode's output.
 static int64_t out_row(int mode, int ef, int k) {
     return mode == PA_OUT_TOPK ? k : static_cast<int64_t>(PA_BEAMS) * ef;
@@ -290,6 +303,8 @@ extern "C" int pa_stage_search_ex(pa_stage *st, const float *host_query, float *
     if (rc != PA_OK || batch == 0) return rc;
     PA_REQUIRE(host_query && host_out_I && host_out_D, "null host pointer");
     PA_REQUIRE(chunk >= 0, "chunk must not be negative");
+    rc = check_alignment(st, mode, nullptr);
+    if (rc != PA_OK) return rc;
     DeviceScope scope;
     PA_CUDA_TRY(scope.enter(st->device));
     // Chunks are what the copies overlap; a launch of the searches below a wave (seven
@@ -334,6 +349,8 @@ extern "C" int pa_stage_search_device_ex(pa_stage *st, const float *dev_query, i
     rc = check_mode(st, mode, ef, k);
     if (rc != PA_OK || batch == 0) return rc;
     PA_REQUIRE(dev_query && dev_out_I && dev_out_D, "null device pointer");
+    rc = check_alignment(st, mode, st->ix.VT == nullptr ? dev_query : nullptr);
+    if (rc != PA_OK) return rc;
     DeviceScope scope;
     PA_CUDA_TRY(scope.enter(st->device));
     int64_t *cand_I = mode == PA_OUT_HANDOFF ? dev_out_I : st->d_out_I;
@@ -454,6 +471,8 @@ extern "C" int pa_stage_submit(pa_stage *st, int slot, const float *host_query, 
     PA_REQUIRE(n == 0 || host_query != nullptr, "null host pointer");
     const int64_t cap = st->slot_rows * PA_BEAMS * st->max_ef;
     if (n > 0) {
+        rc = check_alignment(st, mode, nullptr);
+        if (rc != PA_OK) return rc;
         rc = enqueue_host_chunk(st, host_query,
                                 want_rotated ? st->h_slot_rot + slot * st->slot_rows * st->ix.d_model
                                              : nullptr,

@@ -207,6 +207,61 @@ def test_submit_wait_slots(small_index):
     assert torch.equal(c[0], top_I)
 
 
+def test_unaligned_vectors_are_refused_before_any_launch(small_index):
+    """A stage without a rotation searches the caller's queries as they lie: rows that
+    cannot be read as float4 are refused with nothing enqueued, at batches whose router
+    scores come from either kernel; so are index vectors that do not start on 16 bytes.
+    With a rotation the raw queries may lie anywhere."""
+    from pilotann_b200 import extension
+    from pilotann_b200.stage import SearchStage
+    index, x, q, w = small_index
+    ef, k = 32, 5
+    kept = index.stage._keep
+
+    def shifted(t):
+        out = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape)
+        assert out.copy_(t).data_ptr() % 16 != 0 and out.is_contiguous()
+        return out
+
+    def plain_stage(**other):
+        names = ("packed_nbr", "row_of", "storage", "route_vectors", "entry_nodes", "entry_vectors")
+        return SearchStage(**{**{name: kept[name] for name in names}, **other}, VT=None,
+                           n_neighbors=index.n_neighbors, d_model=w.d_model, max_batch=512, max_ef=64)
+
+    rot = extension.project(q.cuda(), index.VT_cuda).repeat(2, 1)
+    stage = plain_stage()
+    want_I, want_D, _ = index.stage.search_host(q, ef)
+    for batch in (1, 200, 256, 300):
+        before = extension.launch_count()
+        with pytest.raises(RuntimeError, match="16-byte aligned"):
+            stage.search_device(shifted(rot[:batch]), ef)
+        assert extension.launch_count() == before
+        got_I, got_D = stage.search_device(rot[:batch].contiguous(), ef)
+        stage.synchronize()
+        n = min(batch, 256)
+        assert torch.equal(got_I.view(batch, -1)[:n].cpu(), want_I[:n])
+        assert torch.equal(got_D.view(batch, -1)[:n].cpu(), want_D[:n])
+    rot_host = rot.cpu()
+    for name in ("storage", "route_vectors", "entry_vectors"):
+        off = plain_stage(**{name: shifted(kept[name])})
+        for call in (lambda: off.search_device(rot, ef), lambda: off.search_host(rot_host, ef),
+                     lambda: off.submit(0, rot_host[:8].contiguous(), ef)):
+            before = extension.launch_count()
+            with pytest.raises(RuntimeError, match="16-byte aligned"):
+                call()
+            assert extension.launch_count() == before
+        off.close()
+    off = plain_stage()
+    off.attach_refine(shifted(kept["storage_full"]), kept["full_nbr"])
+    with pytest.raises(RuntimeError, match="16-byte aligned"):
+        off.search_device(rot, ef, k=k)
+    off.close()
+    stage.close()
+    raw_I, raw_D = index.stage.search_device(shifted(q.cuda()), ef, k=k)    # rotated first
+    index.stage.synchronize()
+    assert raw_I.shape == (256, k) and torch.isfinite(raw_D).all()
+
+
 def test_ragged_chunks_and_empty_submit(small_index):
     index, x, q, w = small_index
     stage = index.stage
