@@ -12,14 +12,14 @@
 // The dense part -- every query against every router -- is a contraction and
 // runs on the tensor cores when the caller supplies workspace: q.r for all pairs
 // by the tcgen05 GEMM of project.cu (fp32-grade, three TF32 products; small batches by
-// gemm_small_kernel), then
-// score(r) = |r|^2 - 2 q.r.  The tensor-core scores only shortlist: every router
+// its gemm_small_kernel, see route_launch), then
+// score(r) = |r|^2 - 2 q.r.  These scores only shortlist: every router
 // whose score is within a conservative margin of the best one is re-measured
 // exactly (the double-precision sum above), so the id that comes out is the exact
 // one in either mode; normally the shortlist holds a single router.
 //
 // One CTA per query: shortlist + exact re-measure, the winner reduced through
-// shared memory; then each thread owns one leaf.
+// shared memory; then four threads share each leaf.
 #include "pa_common.cuh"
 
 namespace pa {
@@ -200,9 +200,18 @@ int route_launch(int64_t *router, float *leaf_D, int64_t *leaf_I, const float *q
     if (batch == 0) return PA_OK;
     const bool tensor = dots_ws != nullptr && rnorm2 != nullptr && route_vectors != nullptr &&
                         n_routers > 1 && d % 4 == 0 && ldq % 4 == 0;
-    // up to 256 queries by gemm_small_kernel (the scores only shortlist); operands it
-    // cannot read go to the other one, whose tensor map refuses them
-    const bool small = tensor && batch <= 256 && gemm_operands_ok(query, route_vectors, d, ldq, d);
+    // Scores of small batches by gemm_small_kernel (they only shortlist).  It reads the
+    // routers again for every eight queries, so queries x routers decides: up to 2^15 pairs
+    // it is never the slower one, from 256 dimensions on up to 2^16.  Norms, scores and
+    // routing, tensor cores / small kernel, us:
+    //     64 routers, 256 queries (2^14)     128 dimensions 27.6 / 23.5, 768 68.6 / 52.2
+    //     1024 routers, 32 queries (2^15)    96: 25.6 / 25.3, 256: 35.6 / 29.7
+    //     1024 routers, 64 queries (2^16)    96: 25.6 / 27.7, 256: 35.8 / 33.8
+    //     256 routers, 256 queries (2^16)    96: 25.5 / 27.7, 768: 80.9 / 72.4
+    //     1024 routers, 256 queries (2^18)   96: 27.7 / 44.1, 768: 74.8 / 104
+    // Operands it cannot read go to the other one, whose tensor map refuses them.
+    const bool small = tensor && batch <= 256 && batch * n_routers <= (d < 256 ? 1 << 15 : 1 << 16) &&
+                       gemm_operands_ok(query, route_vectors, d, ldq, d);
     if (tensor) {
         const auto scores = small ? gemm_small_launch : gemm_tf32x3_launch;
         int rc = scores(dots_ws, query, route_vectors, static_cast<int>(batch), n_routers, d, ldq,

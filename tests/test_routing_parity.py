@@ -99,10 +99,13 @@ def test_projection_matches_oracle(oracle_lib, B, d, d_out):
 
 
 @pytest.mark.parametrize("n_r,n_l,d,B", [(2, 32, 4, 3), (33, 96, 100, 255), (7, 32, 132, 256),
-                                         (64, 64, 1540, 41), (300, 32, 36, 9)])
+                                         (64, 64, 1540, 41), (300, 32, 36, 9),
+                                         (128, 32, 252, 256), (129, 32, 252, 255),
+                                         (256, 32, 256, 256), (257, 32, 256, 256)])
 def test_routing_of_small_batches(oracle_lib, n_r, n_l, d, B):
-    """Up to 256 queries the router scores come from the kernel for a few rows: odd router
-    counts, dimensions beyond one slice of it, leaves in several passes."""
+    """Small batches have their router scores from the kernel for a few rows: odd router
+    counts, dimensions beyond one slice of it, leaves in several passes, queries x
+    routers on both sides of where the tensor cores take over."""
     from pilotann_b200 import extension
     x, rv, en, ev = _tables(20000, d, n_r, n_l, seed=n_r + d)
     g = torch.Generator().manual_seed(B)
