@@ -222,8 +222,8 @@ void pa_stage_destroy(pa_stage *stage);
  *     (pipeline_cpu.cpp:90-95).
  * The batch is cut into `chunk` queries (0 = one chunk); chunks alternate
  * between the stage's streams so that copy-in, kernels and copy-back overlap.
- * Chunks below a wave of the search kernel (seven queries per SM) are taken
- * together up to one.
+ * As many chunks are taken together as fit a wave of the search kernel (seven
+ * queries per SM); a chunk beyond half a wave stays as it is.
  * Blocks until the handoff is complete.  Host buffers should be pinned. */
 int pa_stage_search(pa_stage *stage, const float *host_query, float *host_rotated,
                     int64_t *host_out_I, float *host_out_D, int64_t batch,

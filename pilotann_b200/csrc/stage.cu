@@ -307,15 +307,20 @@ extern "C" int pa_stage_search_ex(pa_stage *st, const float *host_query, float *
     if (rc != PA_OK) return rc;
     DeviceScope scope;
     PA_CUDA_TRY(scope.enter(st->device));
-    // Chunks are what the copies overlap; a launch of the searches below a wave (seven
-    // queries per SM) takes as long as a whole one, so chunks are taken together up to that
-    // (1024 queries of 768 dimensions at ef 100, chunks of 256, candidates out: 2.14 ms in
-    // four launches on two streams, 1.18 ms in one).
+    // Pieces are what the copies overlap, but pieces of less than a wave of the searches
+    // (seven queries per SM) leave SMs idle: chunks are taken together as long as they do
+    // not exceed one.  Chunks as they come / taken together, us, 148 SMs: 1024 queries of 768
+    // dimensions at ef 100, chunks of 256, candidates out 2128 / 1164, top-k 4814 / 3160; 4096
+    // in chunks of 400 (two together) 6714 / 4476 and 15461 / 12657; 2000 of 96 dimensions at
+    // ef 48 in chunks of 256 1125 / 543 and 2740 / 1094.  Past a wave nothing is gained and the overlap
+    // goes: 2000 in chunks of 1000, apart / together, 536 / 584 and 1096 / 1300.  (Two chunks of
+    // up to half a wave, on a stream each, overlap as they come; taken together they took 0.65 to
+    // 1.10 times as long with candidates out, 0.73 to 1.23 with top-k out, 0.95 and 0.90 on average.)
     if (chunk > 0 && chunk < batch) {
         int sms = 0;
         PA_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, st->device));
         const int64_t wave = 7 * static_cast<int64_t>(sms);
-        if (chunk < wave) chunk *= (wave + chunk - 1) / chunk;
+        if (chunk < wave) chunk *= wave / chunk;
     }
     if (chunk == 0 || chunk > batch) chunk = batch;
     const int64_t d = st->ix.d_model;

@@ -39,7 +39,8 @@ def test_stage_equals_composition_of_ops(small_index, oracle_lib):
                                index.n_neighbors, ef)
     assert torch.equal(I.view(-1, 4, ef), want[0])
     assert torch.equal(D.view(-1, 4, ef), want[1])
-    # chunking and stream count do not change the result
+    # cutting a batch does not change the result (nor where it is really cut: see
+    # test_chunks_beyond_one_wave)
     I2, D2, _ = index.search_candidates(q, ef, chunk_size=0)
     assert torch.equal(I, I2) and torch.equal(D, D2)
 
@@ -267,7 +268,7 @@ def test_ragged_chunks_and_empty_submit(small_index):
     stage = index.stage
     ef, k = 32, 7
     want_I, want_D, _ = stage.search_host(q, ef, k=k)
-    got_I, got_D, _ = stage.search_host(q, ef, chunk=100, k=k)        # 100 + 100 + 56
+    got_I, got_D, _ = stage.search_host(q, ef, chunk=100, k=k)        # taken together: below a wave
     assert torch.equal(want_I, got_I) and torch.equal(want_D, got_D)
     h_I, _, _ = stage.search_host(q, ef, chunk=96)
     h2_I, _, _ = stage.search_host(q, ef)
@@ -280,21 +281,35 @@ def test_ragged_chunks_and_empty_submit(small_index):
 
 
 def test_chunks_beyond_one_wave(small_index):
-    """Chunks are taken together up to a wave of queries; a batch of several waves is still
-    cut, its pieces alternating over the streams: rows as from one launch, in every mode."""
+    """As many chunks as fit a wave of queries are taken together, and no more: a batch of
+    several waves goes in the pieces that the rule names (counted in launches), more of
+    them than the stage has streams, the last one ragged: rows as from one launch, in every mode."""
+    from pilotann_b200 import extension
     index, x, q, w = small_index
-    sms = torch.cuda.get_device_properties(0).multi_processor_count
-    B, ef, k = 2 * 7 * sms + 77, 20, 6
+    wave = 7 * torch.cuda.get_device_properties(0).multi_processor_count
+    B, ef, k = 3 * wave + 300, 20, 6
     many = q.repeat(B // q.size(0) + 1, 1)[:B].contiguous()
     try:
         index.to("cuda", max_batch=B, max_ef=32)
         stage = index.stage
+
+        def launches(n, chunk=0):
+            before = extension.launch_count()
+            stage.search_host(many[:n], ef, chunk=chunk)
+            return extension.launch_count() - before
+
+        for chunk in (100, wave // 3, wave // 2, wave // 2 + 1, wave - 1, wave, wave + 1, 2 * wave):
+            piece = chunk * max(1, wave // chunk)
+            sizes = [min(piece, B - lo) for lo in range(0, B, piece)]
+            assert launches(B, chunk) == sum(launches(n) for n in sizes), (chunk, sizes)
+        assert launches(wave // 2, 50) == launches(wave // 2)             # clipped by the batch
         for mode in ({}, {"stage2": True}, {"k": k}):
             rot = torch.empty(B, q.size(1))
             want_I, want_D, _ = stage.search_host(many, ef, **mode)
-            got_I, got_D, _ = stage.search_host(many, ef, chunk=100, rotated=rot, **mode)
-            assert torch.equal(want_I, got_I) and torch.equal(want_D, got_D)
-            assert torch.equal(got_I[:q.size(0)], got_I[q.size(0):2 * q.size(0)])
+            for chunk in (100, wave // 2 + 1):
+                got_I, got_D, _ = stage.search_host(many, ef, chunk=chunk, rotated=rot, **mode)
+                assert torch.equal(want_I, got_I) and torch.equal(want_D, got_D)
+                assert torch.equal(got_I[:q.size(0)], got_I[q.size(0):2 * q.size(0)])
         assert torch.equal(rot[:q.size(0)], rot[q.size(0):2 * q.size(0)])
     finally:
         index.to("cuda", max_batch=256, max_ef=128)
