@@ -346,6 +346,10 @@ struct RefCtl {
     int n_log;          //          entries admitted
     int st[4];          // expansions and evaluations of the two stages
     int rerun;          //          the query has to be run on the array heaps
+#if PA_REFINE_PROFILE
+    int heap_prof[12];      // thread 0's phases on their way in and out of heap_side
+    long long heap_clock;
+#endif
 };
 constexpr int kAscending = 1;   // the real entries ascend
 constexpr int kHeadStrict = 2;  // the first kSeedHead of them strictly
@@ -953,12 +957,23 @@ __device__ __noinline__ void heap_side(const RefineArgs &A, RefCtl *ctl, int n_s
     __syncwarp();
     int prof[12] = {};
     long long prof_t = 0;
-    if (brief)
+#if PA_REFINE_PROFILE
+    prof_t = ctl->heap_clock;
+#endif
+    if (brief) {
         brief_search<R>(A, S, n_seed, ctl, side, WL, lane, st);
-    else
+        PA_TICK(1);
+    } else {
         heap_loop<R>(A, S, n_seed, seed_lo, max_iter, closed_form, second ? H + seed_lo : 0, ctl,
                      side, WL, lane, st, prof, prof_t);
+    }
     side.finish(second ? S.open + H + 1 : S.buf + 1, H, lane, ctl);
+#if PA_REFINE_PROFILE
+    if (lane == 0) {
+        for (int i = 0; i < 12; ++i) ctl->heap_prof[i] = prof[i];
+        ctl->heap_clock = prof_t;
+    }
+#endif
 }
 
 // The gather warps' half of the general search.
@@ -1145,8 +1160,18 @@ __device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShare
     const bool brief = max_iter == 2 && !speculate && 2 * H >= 32 && G.degree <= 64 &&
                        brief_prepare(S, n_seed, ctl);
     if (w == 0) {
+#if PA_REFINE_PROFILE
+        if (lane == 0) ctl->heap_clock = prof_t;
+        __syncwarp();
+#endif
         heap_side<R>(A, ctl, n_seed, max_iter, second, brief,
                      sorted == (kAscending | kHeadStrict) && n_seed >= H, ctl->st + (second ? 2 : 0));
+#if PA_REFINE_PROFILE
+        if (lane == 0) {
+            for (int i = 0; i < 12; ++i) prof[i] += ctl->heap_prof[i];
+            prof_t = ctl->heap_clock;
+        }
+#endif
     } else if (brief) {
         if (ctl->m1 != ~0ull) {
             gather_node(A, S, G, vis, marker, ctl, S.c_id[ctl->m1 & 0xffffffffu], 0, w - 1, lane, prof, prof_t);

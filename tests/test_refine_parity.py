@@ -10,6 +10,8 @@ full graph, visited marks from the device pool) against
 The handoff both sides consume is produced by the traversal kernel of this
 package on the same tensors.
 """
+import os
+
 import pytest
 import torch
 
@@ -474,6 +476,27 @@ def test_short_residuals(oracle_lib, d, d_p):
                          gpu_order=True, stages=2)
     assert torch.equal(t_I.cpu(), w_I)
     assert torch.equal(t_D.cpu().view(torch.int32), w_D.view(torch.int32))
+
+
+@pytest.mark.skipif("PA_REFINE_PROFILE=1" not in os.environ.get("PILOTANN_B200_DEFINES", ""),
+                    reason="needs a library built with PILOTANN_B200_DEFINES=PA_REFINE_PROFILE=1")
+@pytest.mark.parametrize("ef", [48, 257])
+def test_phases_of_a_profile_build(ef):
+    """What a profile build counts per query: the heap warp's phases (set-up, seed inserts, pops,
+    waiting, inserts, merge, then pushes in units), the gather warp's.  All of them are
+    there and either side's clocks add up to the same time; the result list in registers (ef 48) and the array heaps (ef 257)."""
+    from pilotann_b200 import extension
+    c = _case(n=4000, batch=64, ef=ef)
+    pool = extension.VisitedPool(c["full"].size(0), 64)
+    st = torch.zeros(64, 24, dtype=torch.int32, device="cuda")
+    extension.refine(c["hand_I"], c["hand_D"], c["q_cuda"], c["full_cuda"], c["nbr"], c["row_of"],
+                     c["full_nbr"], pool, ef, c["d_p"], k=10, stats=st)
+    heap, gather = st[:, 4:12].cpu().long(), st[:, 12:].cpu().long()
+    assert (st[:, 2] > 1).all()
+    assert (heap.sum(0) > 0).all(), heap.sum(0)
+    assert (gather[:, [0, 1, 2, 4, 5, 6, 7, 8]].sum(0) > 0).all(), gather.sum(0)   # (3: long rows)
+    whole = heap[:, :7].sum(1).double() / gather.sum(1).double()
+    assert (whole > 0.8).all() and (whole < 1.25).all()
 
 
 def test_replay_of_upstream_fixtures():
