@@ -331,6 +331,21 @@ __device__ __forceinline__ void warp_sort(float (&k)[E], int32_t (&v)[E], int la
     }
 }
 
+// Whether an entry of a heap of 32 E nodes equals its parent or its left sibling (one lane's
+// answer for its nodes lane * E + 1 ..): where equal keys are common, some are that close.
+template <int E, class Key>
+__device__ __forceinline__ bool heap_shows_twins(const float (&k)[E], const int32_t (&v)[E], int lane,
+                                                 Key key_of) {
+    bool twins = false;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int node = lane * E + e + 1;
+        if (node > 1 && v[e] >= 0)
+            twins = twins || k[e] == key_of(node >> 1) || ((node & 1) != 0 && k[e] == key_of(node - 1));
+    }
+    return twins;
+}
+
 // Whether two neighbours of the sorted entries from position `from` on (or the first of
 // them and the one in front of it) have equal keys; empty entries (id -1) are alike.
 template <int E>
