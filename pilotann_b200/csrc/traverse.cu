@@ -935,12 +935,13 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
     // stores.  With pairwise different keys that is the heap in ascending order: warp b
     // sorts beam b in registers.  Equal keys among the entries that come out: the layout
     // of the heap decides, and the result warp pops them one by one, H dependent heap
-    // operations; where an entry equals its parent or its sibling, they are popped at once
-    // without the sort.  Popping always, 1024 queries took (us) 431, 1946 and 522 instead of
-    // 408, 1894 and 484 (96 dimensions at ef 256, 200 at 192, 2000 of 96 at 128); with every vector
-    // there 40 times, 8192 of 96 dimensions at ef 128 507 popping always, 584 sorting first, 508 now.
+    // operations; a beam whose heap shows equal keys is not sorted first.  Popping always, 1024
+    // queries took (us) 431, 1946 and 522 instead of 408, 1894 and 484 (96 dimensions at ef 256,
+    // 200 at 192, 2000 of 96 at 128); with every vector there 40 times, 8192 of 96 dimensions
+    // at ef 128 507 popping always, 575 sorting first, 500 now, at ef 256 869, 976 and 804.
     const int n_discard = max(H - ef, 0), n_real = min(ef, H);
-    bool popped;  // CTA-uniform
+    if (threadIdx.x == 0) again_s[0] = 0;
+    __syncthreads();
     {
         float k[H / 32];
         int32_t v[H / 32];
@@ -949,18 +950,20 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
             k[e] = res_key[w][lane * (H / 32) + e];
             v[e] = res_id[w][lane * (H / 32) + e];
         }
-        popped = __syncthreads_or(heap_shows_twins(k, v, lane, [&](int node) { return res_key[w][node - 1]; }));
-        if (!popped) {
+        if (heap_shows_twins<H / 32>(lane, [&](int node) { return res_key[w][node - 1]; })) {
+            again_s[0] = 1;
+        } else {
             warp_sort(k, v, lane);
+            if (warp_has_twins(k, v, n_discard, lane)) again_s[0] = 1;
 #pragma unroll
             for (int e = 0; e < H / 32; ++e) {
                 const int i = lane * (H / 32) + e - n_discard;
                 if (i >= 0) open_val[w][i] = make_int2(v[e], __float_as_int(-k[e]));
             }
-            popped = __syncthreads_or(warp_has_twins(k, v, n_discard, lane));
         }
     }
-    if (w == 1 && popped) {
+    __syncthreads();
+    if (w == 1 && again_s[0] != 0) {
         for (int p = 0; p < n_discard + n_real; ++p) {
             const float key = rkey[0];
             const int32_t id = rid[0];
@@ -1272,14 +1275,14 @@ traverse_wide_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ 
     if (results) {
         float k[H / 32];
         int32_t v[H / 32];
-#pragma unroll
-        for (int x = 0; x < H / 32; ++x) {
-            const HeapEntry r = res[1 + lane * (H / 32) + x];
-            k[x] = r.k;
-            v[x] = r.v;
-        }
-        bool popped = __any_sync(kAll, heap_shows_twins(k, v, lane, [&](int node) { return res[node].k; }));
+        bool popped = heap_shows_twins<H / 32>(lane, [&](int node) { return res[node].k; });
         if (!popped) {
+#pragma unroll
+            for (int x = 0; x < H / 32; ++x) {
+                const HeapEntry r = res[1 + lane * (H / 32) + x];
+                k[x] = r.k;
+                v[x] = r.v;
+            }
             warp_sort(k, v, lane);
             popped = warp_has_twins(k, v, n_discard, lane);
         }

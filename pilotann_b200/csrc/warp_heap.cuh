@@ -144,7 +144,8 @@ template <int W> struct PathBits {
         for (int i = 0; i < kUniform; ++i) w[i] = 0;
         deep = 0;
     }
-    __device__ __forceinline__ void build_larger(const HeapEntry *h, int n, int lane) {
+    template <bool kLarger>
+    __device__ __forceinline__ void build(const HeapEntry *h, int n, int lane) {
         deep = 0;
 #pragma unroll
         for (int i = 0; i < W; ++i) {
@@ -152,12 +153,19 @@ template <int W> struct PathBits {
             bool right = false;
             if (node >= 1 && 2 * node + 1 <= n) {
                 const int4 p = *reinterpret_cast<const int4 *>(h + 2 * node);
-                right = __int_as_float(p.z) > __int_as_float(p.x);
+                const float lk = __int_as_float(p.x), rk = __int_as_float(p.z);
+                right = kLarger ? rk > lk : rk < lk;
             }
             const uint32_t word = __ballot_sync(kAll, right);
             if (i < kUniform) w[i < kUniform ? i : 0] = word;
             else if (lane == i) deep = word;
         }
+    }
+    __device__ __forceinline__ void build_larger(const HeapEntry *h, int n, int lane) {
+        build<true>(h, n, lane);
+    }
+    __device__ __forceinline__ void build_smaller(const HeapEntry *h, int n, int lane) {
+        build<false>(h, n, lane);
     }
     // The leaf at the end of the path in a heap of n nodes.  All nodes of the first kSure
     // levels below the root exist for every n that comes with this many words.
@@ -331,19 +339,19 @@ __device__ __forceinline__ void warp_sort(float (&k)[E], int32_t (&v)[E], int la
     }
 }
 
-// Whether an entry of a heap of 32 E nodes equals its parent or its left sibling (one lane's
-// answer for its nodes lane * E + 1 ..): where equal keys are common, some are that close.
+// Whether a heap of 32 E nodes shows entries equal to their parents (empty ones, -inf, aside), in
+// two lanes at least: a single pair is chance, and where equal keys are common many stand
+// so, since a sinking key stops above its equal.
 template <int E, class Key>
-__device__ __forceinline__ bool heap_shows_twins(const float (&k)[E], const int32_t (&v)[E], int lane,
-                                                 Key key_of) {
+__device__ __forceinline__ bool heap_shows_twins(int lane, Key key_of) {
     bool twins = false;
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-        const int node = lane * E + e + 1;
-        if (node > 1 && v[e] >= 0)
-            twins = twins || k[e] == key_of(node >> 1) || ((node & 1) != 0 && k[e] == key_of(node - 1));
+        const int node = 32 * e + lane + 1;
+        const float k = key_of(node);
+        twins = twins || (node > 1 && k == key_of(max(node >> 1, 1)) && k > -CUDART_INF_F);
     }
-    return twins;
+    return __popc(__ballot_sync(kAll, twins)) >= 2;
 }
 
 // Whether two neighbours of the sorted entries from position `from` on (or the first of
