@@ -39,8 +39,8 @@
 //     result; it lives in shared memory, stored 1-based as {key, id} pairs so that
 //     both children of a node come in one 16-byte load, and is driven by the 32
 //     lanes of the heap warp together (see the routines below).  So does the result
-//     heap (H entries) where H > 256; up to there the results are a sorted list in
-//     registers (TopList);
+//     heap (H entries) where H > 256, and for queries with several equal distances or a
+//     NaN (finish_query); the others' results are a sorted list in registers (TopList);
 //   * H follows upstream's CPU dispatch (traverse_cpu.cpp:228-254);
 //   * exact visited marks (extension/inc/bitmask.hpp:12-45) shared by the two
 //     stages of a query, as upstream shares one marker between them;
@@ -188,6 +188,9 @@ template <int R> struct TopList {
         }
     }
 };
+
+// Words of comparison bits of a result heap where the open heap, twice as large, has R.
+__host__ __device__ constexpr int result_words(int R) { return R >= 4 ? R / 2 : 1; }
 
 // Registers per lane of the list for a capacity of H; 0: the array heap is used.
 __host__ __device__ constexpr int list_regs_for(int H) {
@@ -346,13 +349,18 @@ struct RefCtl {
     int n_log;          //          entries admitted
     int st[4];          // expansions and evaluations of the two stages
     int rerun;          //          the query has to be run on the array heaps
+    int half;           // the first stage stands, the second shall be run on the array heaps
+    int tied;           // equal neighbours in the first stage's output, where its merge gave up
 #if PA_REFINE_PROFILE
     int heap_prof[12];      // thread 0's phases on their way in and out of heap_side
     long long heap_clock;
+    int phases[2][12];      // of threads 0 and 32 on their way to finish_query
+    long long clock[2];
 #endif
 };
 constexpr int kAscending = 1;   // the real entries ascend
 constexpr int kHeadStrict = 2;  // the first kSeedHead of them strictly
+constexpr int kManyTied = 2;    // RefCtl::tied from which on more are expected
 constexpr int kSeedHead = 26;   // entries the seeding of the open heap may look at
 
 // Every thread of the CTA, whichever side of the warp specialisation it is on.
@@ -461,7 +469,7 @@ __device__ __forceinline__ void gather_node(const RefineArgs &A, const RefShared
 // that matter, or a distance that is negative or NaN, make the outcome depend on
 // upstream's exact sequence: nothing is written then and the caller runs that
 // sequence.  Returns true (CTA-uniform) if the output is written.
-template <int R>
+template <bool kList>
 __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, int seed_lo,
                                                    int n_seed, int n_real, int k_out, int n_check,
                                                    RefCtl *ctl) {
@@ -471,7 +479,7 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
     // the array heap holds negated distances, the dumped list distances
     auto result_at = [&](int x) {
         HeapEntry e = S.buf[1 + x];
-        if (R == 0) e.k = -e.k;
+        if (!kList) e.k = -e.k;
         return e;
     };
     const int N = H + n_seed - seed_lo;
@@ -562,7 +570,7 @@ __device__ __forceinline__ bool select_sort_output(const RefShared &S, int H, in
             __syncthreads();
         }
     }
-    bool tie = R > 0 && ctl->amb < CUDART_INF_F && ctl->amb <= a[n_check - 1].k;
+    bool tie = kList && ctl->amb < CUDART_INF_F && ctl->amb <= a[n_check - 1].k;
     for (int i = tid; i < n_check && i + 1 < H; i += n_thr)
         if (a[i].k == a[i + 1].k && (a[i].v >= 0 || a[i + 1].v >= 0)) tie = true;
     if (tie) ctl->tie = 1;
@@ -635,7 +643,7 @@ extern __shared__ __align__(16) unsigned char ref_smem[];
 
 // The heap warp's side of a stage: the result list (or the array heap, R = 0), the
 // log, the counters.
-template <int R> struct HeapSide {
+template <int R, bool kList> struct HeapSide {
     TopList<R> top;
     float worst;
     int n_log;
@@ -705,7 +713,56 @@ template <int R> struct HeapSide {
     }
 };
 
-template <> struct HeapSide<0> {
+// Array heaps with the comparison bits of both: a stage that will meet equal distances
+// (finish_query).  (The bits follow the array as long as no key is NaN.)
+template <int R> struct HeapSide<R, false> {
+    float worst;
+    PathBits<R> larger;                 // of the open heap
+    PathBits<result_words(R)> smaller;  // of the result heap
+
+    __device__ __forceinline__ void clear(int, int) {
+        worst = CUDART_INF_F;
+        smaller.clear();
+    }
+    __device__ __forceinline__ void open_filled(const RefShared &S, int n, int lane) {
+        larger.build_larger(S.open, n, lane);
+    }
+    __device__ __forceinline__ void open_push(const RefShared &S, int n, float k, int32_t v,
+                                              int lane, const WalkLane &) {
+        bit_replace(S.open, n, k, v, larger, lane);
+    }
+    __device__ __forceinline__ HeapEntry open_pop(const RefShared &S, int n, int lane,
+                                                  const WalkLane &WL) {
+        return bit_pop(S.open, n, larger, lane, WL);
+    }
+    __device__ __forceinline__ float worst_of(const RefShared &) const { return worst; }
+    template <class F>
+    __device__ __forceinline__ void admit(const RefShared &S, const int32_t *nb_id,
+                                          const float *nb_d, int n_new, int, int H, int lane,
+                                          const WalkLane &, RefCtl *ctl, F f) {
+        for (int c = 0; c < n_new; c += 32) {
+            const bool in = c + lane < n_new;
+            const float dist = in ? nb_d[c + lane] : CUDART_INF_F;
+            const int32_t id = in ? nb_id[c + lane] : -1;
+            if (!(dist >= 0.0f)) ctl->rerun = 1;  // NaN: see search_stage
+            unsigned ahead = kAll;
+            for (;;) {
+                const unsigned m = __ballot_sync(kAll, dist < worst) & ahead;
+                if (m == 0) break;
+                const int j = __ffs(m) - 1;
+                ahead = 0xfffffffeu << j;
+                const float nk = __shfl_sync(kAll, dist, j);
+                const int32_t nv = __shfl_sync(kAll, id, j);
+                bit_sink(S.buf, H, HeapEntry{-nk, nv}, smaller, lane);
+                worst = -S.buf[1].k;
+                f(nk, nv, c + j);
+            }
+        }
+    }
+    __device__ __forceinline__ void finish(HeapEntry *, int, int, RefCtl *) {}
+};
+
+template <> struct HeapSide<0, false> {
     __device__ __forceinline__ void clear(int, int) {}
     __device__ __forceinline__ void open_filled(const RefShared &, int, int) {}
     __device__ __forceinline__ void open_push(const RefShared &S, int n, float k, int32_t v,
@@ -794,9 +851,9 @@ __device__ __forceinline__ bool brief_prepare(const RefShared &S, int n_seed, Re
 }
 
 // The heap warp's half; the gather warps run the two expansions (search_stage).
-template <int R>
+template <int R, bool kList>
 __device__ __forceinline__ void brief_search(const RefineArgs &A, const RefShared &S, int n_seed,
-                                             RefCtl *ctl, HeapSide<R> &side, const WalkLane &WL,
+                                             RefCtl *ctl, HeapSide<R, kList> &side, const WalkLane &WL,
                                              int lane, int *st) {
     constexpr unsigned long long kNone = ~0ull;
     const int H = A.H;
@@ -862,10 +919,10 @@ __device__ __forceinline__ void brief_search(const RefineArgs &A, const RefShare
 }
 
 // The heap warp's half of the general search (:64-136).
-template <int R>
+template <int R, bool kList>
 __device__ __forceinline__ void heap_loop(const RefineArgs &A, const RefShared &S, int n_seed,
                                           int seed_lo, int max_iter, bool closed_form, int log_room,
-                                          RefCtl *ctl, HeapSide<R> &side, const WalkLane &WL,
+                                          RefCtl *ctl, HeapSide<R, kList> &side, const WalkLane &WL,
                                           int lane, int *st, int *prof, long long &prof_t) {
     (void)prof; (void)prof_t;
     const int H = A.H;
@@ -943,14 +1000,14 @@ __device__ __forceinline__ void heap_loop(const RefineArgs &A, const RefShared &
 // The heap warp's half of a stage.  Out of line: the registers of its heaps and those
 // of the gather's row loads are never live together, and inlined they were allocated as
 // if they were (rows spilled, 768 dimensions 17.8 instead of 16.1 ms per 8192 queries).
-template <int R>
+template <int R, bool kList>
 __device__ __noinline__ void heap_side(const RefineArgs &A, RefCtl *ctl, int n_seed, int max_iter,
                                        bool second, bool brief, bool closed_form, int *st) {
     const RefShared S = ref_shared(A, ref_smem);
     const int lane = threadIdx.x & 31, H = A.H;
     const int seed_lo = second ? max(n_seed - H, 0) : 0;
     const WalkLane WL = walk_lane(lane);
-    HeapSide<R> side;
+    HeapSide<R, kList> side;
     side.clear(H, lane);
     ctl->amb = CUDART_INF_F;  // all lanes alike
     st[0] = st[1] = 0;
@@ -961,10 +1018,10 @@ __device__ __noinline__ void heap_side(const RefineArgs &A, RefCtl *ctl, int n_s
     prof_t = ctl->heap_clock;
 #endif
     if (brief) {
-        brief_search<R>(A, S, n_seed, ctl, side, WL, lane, st);
+        brief_search<R, kList>(A, S, n_seed, ctl, side, WL, lane, st);
         PA_TICK(1);
     } else {
-        heap_loop<R>(A, S, n_seed, seed_lo, max_iter, closed_form, second ? H + seed_lo : 0, ctl,
+        heap_loop<R, kList>(A, S, n_seed, seed_lo, max_iter, closed_form, second ? H + seed_lo : 0, ctl,
                      side, WL, lane, st, prof, prof_t);
     }
     side.finish(second ? S.open + H + 1 : S.buf + 1, H, lane, ctl);
@@ -1017,14 +1074,13 @@ __device__ __forceinline__ void gather_loop(const RefineArgs &A, const RefShared
 }
 
 // Upstream's sequence at the end of a stage (:139-162), by the heap warp.
-template <int R>
+template <int R, bool kList>
 __device__ __noinline__ void upstream_output(const RefineArgs &A, const RefCtl *ctl, int n_seed,
                                              int n_real, int k_out, bool second) {
-    constexpr int kReplayWords = R >= 4 ? R / 2 : 1;
     const RefShared S = ref_shared(A, ref_smem);
     const int lane = threadIdx.x & 31, H = A.H;
     const int seed_lo = second ? max(n_seed - H, 0) : 0;
-    PathBits<kReplayWords> smaller;
+    PathBits<result_words(R)> smaller;
     const WalkLane WL = walk_lane(lane);
     auto push = [&](float dist, int32_t id) {
         if (R == 0) warp_pushpop(S.buf, H, -dist, id, lane, WL);
@@ -1038,7 +1094,8 @@ __device__ __noinline__ void upstream_output(const RefineArgs &A, const RefCtl *
         bit_sink(S.buf, H, HeapEntry{CUDART_INF_F, -1}, smaller, lane);
         return out;
     };
-    if (R > 0) {
+    if (R > 0 && !kList) smaller.build_smaller(S.buf, H, lane);
+    if (kList) {
         // the result heap as upstream's pushes leave it; the log's part in buf makes
         // room for it by going where the list was
         HeapEntry *moved = S.open;
@@ -1085,7 +1142,7 @@ __device__ __noinline__ void upstream_output(const RefineArgs &A, const RefCtl *
 // evaluations through ctl->st, and false (CTA-uniform) if the query
 // has to be run on the array heaps (R > 0 only: a NaN distance, of a neighbour or of a
 // seed, which upstream's tests let into the heaps, or equal distances after more admissions than the log holds).
-template <int R>
+template <int R, bool kList>
 __device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShared &S,
                                              const RefGraph &G, uint8_t *vis, uint8_t marker,
                                              int n_seed, int from, int max_iter, int k_out,
@@ -1139,7 +1196,7 @@ __device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShare
     }
     PA_GTICK(4);  // residual distances of the seeds
     // :65-68
-    if (R == 0)
+    if (!kList)
         for (int i = tid; i < H + 2; i += blockDim.x) S.buf[i] = HeapEntry{-CUDART_INF_F, -1};
     for (int i = tid; i < 2 * H + 2; i += blockDim.x) S.open[i] = HeapEntry{CUDART_INF_F, -1};
     // :69-79, the marks (their order does not matter; the heap inserts below keep it)
@@ -1164,7 +1221,7 @@ __device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShare
         if (lane == 0) ctl->heap_clock = prof_t;
         __syncwarp();
 #endif
-        heap_side<R>(A, ctl, n_seed, max_iter, second, brief,
+        heap_side<R, kList>(A, ctl, n_seed, max_iter, second, brief,
                      sorted == (kAscending | kHeadStrict) && n_seed >= H, ctl->st + (second ? 2 : 0));
 #if PA_REFINE_PROFILE
         if (lane == 0) {
@@ -1193,22 +1250,26 @@ __device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShare
     // left comes out worst first and is stored ascending
     const int n_real = min(k_out, H);
     const bool done =  // CTA-uniform
-        R > 0 && second
+        kList && second
             ? merge_sorted_output(S, list, H, seed_lo, n_seed, n_real, k_out, ctl)
-            : select_sort_output<R>(S, H, seed_lo, n_seed, n_real, k_out, min(n_check, n_real), ctl);
-    if (tid == 0) ctl->sorted = kAscending | kHeadStrict;  // select_sort_output has seen to it
+            : select_sort_output<kList>(S, H, seed_lo, n_seed, n_real, k_out, min(n_check, n_real), ctl);
+    if (tid == 0) {
+        ctl->sorted = kAscending | kHeadStrict;  // select_sort_output has seen to it
+        if (!second) ctl->tied = 0;
+    }
     if (!done) {
-        if (R > 0 && second && ctl->n_log > log_room) return false;
-        if (w == 0) upstream_output<R>(A, ctl, n_seed, n_real, k_out, second);
+        if (kList && second && ctl->n_log > log_room) return false;
+        if (w == 0) upstream_output<R, kList>(A, ctl, n_seed, n_real, k_out, second);
         __syncthreads();
         // NaN distances may come out in any order; equal ones near the front forbid the
         // closed form of the next stage's seeding (pads are not seeded)
         for (int i = tid; i + 1 < n_real; i += blockDim.x) {
             const int at = k_out - n_real + i;
             if (!(S.c_d[at] <= S.c_d[at + 1])) ctl->sorted = 0;
-            else if (i < kSeedHead && S.c_d[at] == S.c_d[at + 1] &&
-                     (S.c_id[at] >= 0 || S.c_id[at + 1] >= 0))
-                atomicAnd(&ctl->sorted, kAscending);
+            else if (S.c_d[at] == S.c_d[at + 1] && (S.c_id[at] >= 0 || S.c_id[at + 1] >= 0)) {
+                if (i < kSeedHead) atomicAnd(&ctl->sorted, kAscending);
+                if (!second) atomicAdd(&ctl->tied, 1);
+            }
         }
     }
     // pops of an exhausted heap give (-1, key +inf): the leading pads
@@ -1222,16 +1283,28 @@ __device__ __forceinline__ bool search_stage(const RefineArgs &A, const RefShare
     return true;
 }
 
-// Query b from its candidates to its output.  False: see search_stage.
-template <int R>
-__device__ __forceinline__ bool run_query(const RefineArgs &A, const RefShared &S, int64_t b,
-                                          int slot, uint8_t *vis, RefCtl *ctl) {
+// A stage of the running query, with the arguments that go with it.
+template <int R, bool kList>
+__device__ __forceinline__ bool query_stage(const RefineArgs &A, const RefShared &S, uint8_t *vis,
+                                            int marker, bool second, RefCtl *ctl, int *prof,
+                                            long long &prof_t) {
+    // sub-graph, REFINE_STEP expansions (traverse_cpu.cpp:317-326); full graph, same marker
+    // (:327-336)
+    return search_stage<R, kList>(
+        A, S, second ? A.full : A.sub, vis, static_cast<uint8_t>(marker), A.n_cand, second ? A.d : A.d_p,
+        min(second ? 1024 : 2, 2 * A.ef), second ? A.k : A.n_cand, second,
+        second ? A.k : A.stages >= 3 ? max(A.k, kSeedHead) : A.H, ctl, prof, prof_t);
+}
+
+// Query b is loaded and gets a marker of its own.
+__device__ __forceinline__ int begin_query(const RefineArgs &A, const RefShared &S, int64_t b,
+                                           int slot, uint8_t *vis, RefCtl *ctl) {
     const int tid = threadIdx.x;
     // next marker of this slot; the array is wiped when the markers run out
     // (bitmask.hpp:17-36 does the same on wrap-around)
     if (tid == 0) {
         ctl->marker = A.epoch[slot] + 1;
-        ctl->rerun = 0;
+        ctl->rerun = ctl->half = 0;
         ctl->st[2] = ctl->st[3] = 0;
     }
     __syncthreads();
@@ -1243,7 +1316,7 @@ __device__ __forceinline__ bool run_query(const RefineArgs &A, const RefShared &
         marker = 1;
     }
     __syncthreads();
-    if (tid == 0) A.epoch[slot] = marker;
+    if (tid == 0) A.epoch[slot] = ctl->marker = marker;
 
     for (int i = tid; i < A.d; i += blockDim.x) S.q[i] = A.query[b * A.ldq + i];
     for (int i = tid; i < A.n_cand; i += blockDim.x) {
@@ -1252,21 +1325,14 @@ __device__ __forceinline__ bool run_query(const RefineArgs &A, const RefShared &
         S.c_d[i] = A.cand_D[b * A.n_cand + i];
     }
     __syncthreads();
-    int prof[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-    long long prof_t = 0;
-#if PA_REFINE_PROFILE
-    prof_t = pinned_clock();
-#endif
-    // stage 2 (traverse_cpu.cpp:317-326): sub-graph, REFINE_STEP expansions
+    return marker;
+}
+
+__device__ __forceinline__ void end_query(const RefineArgs &A, const RefShared &S, int64_t b,
+                                          const RefCtl *ctl, const int *prof) {
+    (void)prof;
+    const int tid = threadIdx.x;
     const int k_last = A.stages >= 3 ? A.k : A.n_cand;
-    if (!search_stage<R>(A, S, A.sub, vis, static_cast<uint8_t>(marker), A.n_cand, A.d_p,
-                         min(2, 2 * A.ef), A.n_cand, false, A.stages >= 3 ? max(A.k, kSeedHead) : A.H,
-                         ctl, prof, prof_t))
-        return false;
-    if (A.stages >= 3 &&  // stage 3 (:327-336): full graph, same marker
-        !search_stage<R>(A, S, A.full, vis, static_cast<uint8_t>(marker), A.n_cand, A.d,
-                         min(1024, 2 * A.ef), A.k, true, A.k, ctl, prof, prof_t))
-        return false;
     for (int i = tid; i < k_last; i += blockDim.x) {
         A.out_I[b * k_last + i] = S.c_id[i];
         A.out_D[b * k_last + i] = S.c_d[i];
@@ -1284,15 +1350,69 @@ __device__ __forceinline__ bool run_query(const RefineArgs &A, const RefShared &
         for (int i = 0; i < 4; ++i) A.stats[b * 4 + i] = ctl->st[i];
 #endif
     }
+}
+
+// Query b from its candidates to its output.  False: finish_query has to.
+template <int R>
+__device__ __forceinline__ bool run_query(const RefineArgs &A, const RefShared &S, int64_t b,
+                                          int slot, uint8_t *vis, RefCtl *ctl) {
+    const int marker = begin_query(A, S, b, slot, vis, ctl);
+    int prof[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    long long prof_t = 0;
+#if PA_REFINE_PROFILE
+    prof_t = pinned_clock();
+#endif
+    if (!query_stage<R, (R > 0)>(A, S, vis, marker, false, ctl, prof, prof_t)) return false;
+    if (A.stages >= 3) {
+        if (R > 0 && ctl->tied >= kManyTied) {
+#if PA_REFINE_PROFILE
+            if (threadIdx.x == 0 || threadIdx.x == 32) {
+                ctl->clock[threadIdx.x / 32] = prof_t;
+                for (int i = 0; i < 12; ++i) ctl->phases[threadIdx.x / 32][i] = prof[i];
+            }
+#endif
+            if (threadIdx.x == 0) ctl->half = 1;
+            return false;
+        }
+        if (!query_stage<R, (R > 0)>(A, S, vis, marker, true, ctl, prof, prof_t)) return false;
+    }
+    end_query(A, S, b, ctl, prof);
     return true;
 }
 
-// The way back to the array heaps, out of line: it has hardly ever work to do.
-__device__ __noinline__ void run_query_again(const RefineArgs &A, int64_t b, RefCtl *ctl) {
+// What is left of a query for the array heaps in a kernel that has the list, out of line: few
+// queries need it.  With comparison bits the second stage of a query whose first stage met
+// several equal distances, since the second will meet more of them, and with the list each tie
+// ends in a replay of the log by one warp or, when the log is full, in a second run of the
+// query.  (One equal pair is chance as a rule and stays with the list: 1024 queries at ef 128 and
+// k 100 in 300 k different vectors of 200 dimensions 2180 us, with every tied one here 2330.)
+// Without: both stages of a query that met a NaN or overflowed the log.  The whole search where
+// every vector is there twice (300 k), us, heaps only / list only / now: 1024 queries of 96
+// dimensions at ef 256 3379 / 5418 / 2820, 8192 at ef 128 8934 / 11392 / 8325; of 200 dimensions
+// 1024 at ef 128 2665 / 3736 / 2521, 8192 at ef 32 5768 / 9144 / 6164.  (Called from one place, at
+// the end of the query: a call between the stages cost a lone query 2 % in spills around it.)
+template <int R>
+__device__ __noinline__ void finish_query(const RefineArgs &A, int64_t b, RefCtl *ctl) {
     __syncthreads();
     const RefShared S = ref_shared(A, ref_smem);
     const int slot = A.slot_begin + blockIdx.x;
-    run_query<0>(A, S, b, slot, A.marks + static_cast<int64_t>(slot) * A.slot_stride, ctl);
+    uint8_t *vis = A.marks + static_cast<int64_t>(slot) * A.slot_stride;
+    if (ctl->half != 0) {
+        int prof[12] = {};
+        long long prof_t = 0;
+#if PA_REFINE_PROFILE
+        if (threadIdx.x == 0 || threadIdx.x == 32) {
+            prof_t = ctl->clock[threadIdx.x / 32];
+            for (int i = 0; i < 12; ++i) prof[i] = ctl->phases[threadIdx.x / 32][i];
+        }
+#endif
+        if (query_stage<R, false>(A, S, vis, ctl->marker, true, ctl, prof, prof_t)) {
+            end_query(A, S, b, ctl, prof);
+            return;
+        }
+        __syncthreads();
+    }
+    run_query<0>(A, S, b, slot, vis, ctl);
 }
 
 template <int R, int kMaxThreads, int kMinCtas>
@@ -1307,7 +1427,7 @@ __global__ void __launch_bounds__(kMaxThreads, kMinCtas) refine_kernel(const __g
     // CTA i starts on query i; whoever finishes claims the next unclaimed query (queries
     // differ several-fold in length, and a launch is over when its last CTA is)
     for (int64_t b = blockIdx.x; b < A.batch;) {
-        if (!run_query<R>(A, S, b, slot, vis, ctl)) run_query_again(A, b, ctl);
+        if (!run_query<R>(A, S, b, slot, vis, ctl)) finish_query<R>(A, b, ctl);
         if (tid == 0) ctl->next = atomicAdd(A.claim, 1u);
         __syncthreads();
         b = static_cast<int64_t>(gridDim.x) + ctl->next;

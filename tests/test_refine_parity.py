@@ -478,6 +478,178 @@ def test_short_residuals(oracle_lib, d, d_p):
     assert torch.equal(t_D.cpu().view(torch.int32), w_D.view(torch.int32))
 
 
+def _on_array_heaps(ids, dist, q, full, sub, graph, k, ef, H, d_p):
+    """The refinement of one query with upstream's array heaps in the comparisons of the
+    kernel's (they differ from the oracle's for NaN only), the node it prepares ahead
+    included: with NaN in the open heap that is not always the one popped next, and its
+    neighbours stay marked.  Returns what both stages leave, expansions and evaluations, and
+    the most results a stage admitted."""
+    inf = float("inf")
+
+    def sink(h, me):
+        n, c = len(h), 0
+        while 2 * c + 1 < n:
+            child = 2 * c + 1
+            if child + 1 < n and h[child + 1][0] < h[child][0]:
+                child += 1
+            if not h[child][0] < me[0]:
+                break
+            h[c], c = h[child], child
+        h[c] = me
+
+    def pop(h):
+        out = h[0]
+        sink(h, (inf, -1))
+        return out
+
+    def pushpop(h, key, v):
+        if not key <= h[0][0]:
+            sink(h, (key, v))
+
+    def replace(h, key, v):
+        n, c = len(h), 0
+        while 2 * c + 1 < n:
+            child = 2 * c + 1
+            if child + 1 < n and h[child + 1][0] > h[child][0]:
+                child += 1
+            c = child
+        if key >= h[c][0]:
+            return
+        while c > 0 and h[(c - 1) // 2][0] > key:
+            h[c], c = h[(c - 1) // 2], (c - 1) // 2
+        h[c] = (key, v)
+
+    visited, stats, admitted = set(), [], 0
+
+    def stage(seeds, csr, max_iter, k_out, ahead):
+        nonlocal admitted
+        res, open_ = [(-inf, -1)] * H, [(inf, -1)] * (2 * H)
+        for v, key in seeds:
+            if v >= 0:
+                visited.add(v)
+                replace(open_, key, v)
+
+        def gather(u):
+            row = [v for v in csr[1][csr[0][u]:csr[0][u + 1]].tolist() if v not in visited]
+            visited.update(row)
+            return [(((q - full[v]) ** 2).sum().item(), v) for v in row]
+
+        n_expand = n_eval = n_push = 0
+        key, u = pop(open_)
+        guess = None
+        for step in range(max_iter):
+            if u < 0 or key >= -res[0][0]:
+                break
+            if guess is None or guess[0] != u:
+                guess = (u, gather(u))
+            new, root = guess[1], open_[0]
+            n_expand += 1
+            n_eval += len(new)
+            for dv, v in new:
+                if not dv >= -res[0][0]:
+                    pushpop(res, -dv, v)
+                    replace(open_, dv, v)
+                    n_push += 1
+            guess = None
+            if step + 1 < max_iter:
+                if ahead:
+                    best = min((x for x in new if x[0] < inf), key=lambda x: x[0], default=(inf, -1))
+                    at = best[1] if best[0] < root[0] else root[1]
+                    guess = (at, gather(at)) if at >= 0 else None
+                key, u = pop(open_)
+        admitted = max(admitted, n_push)
+        stats.extend((n_expand, n_eval))
+        for v, key in seeds:
+            if v >= 0:
+                pushpop(res, -key, v)
+        for _ in range(k_out, H):
+            pop(res)
+        out = [pop(res) for _ in range(k_out)][::-1]
+        return [(v, -key) for key, v in out]
+
+    seeds = [(v, dv + ((q[d_p:] - full[v][d_p:]) ** 2).sum().item() if v >= 0 else dv)
+             for v, dv in zip(ids.tolist(), dist.tolist())]
+    first = stage(seeds, sub, min(2, 2 * ef), len(seeds), False)
+    last = stage(first, graph, min(1024, 2 * ef), k, True)
+    return first, last, stats, admitted
+
+
+@pytest.mark.parametrize("ef,k,n_cand,spoil", [
+    (48, 10, 192, "seed distance"), (96, 20, 384, "seed distance"), (192, 10, 768, "seed distance"),
+    (64, 10, 256, "seed vector"), (128, 60, 512, "seed vector"), (256, 10, 1024, "seed vector"),
+    (30, 10, 120, "neighbour"), (100, 10, 400, "neighbour"), (150, 30, 600, "neighbour"),
+    (257, 10, 1028, "seed distance"), (257, 10, 1028, "seed vector"), (257, 10, 1028, "neighbour"),
+    (48, 40, 40, "twins"), (100, 60, 60, "twins"), (192, 90, 92, "twins"), (257, 60, 60, "twins"),
+    (48, 10, 40, "unsampled twins"), (100, 10, 60, "unsampled twins"),
+    (192, 10, 92, "unsampled twins")])
+def test_queries_sent_back_to_the_array_heaps(ef, k, n_cand, spoil):
+    """What makes a query leave the result list for the array heaps, for each width of the
+    list and for the heaps alone (ef 257): a NaN among the seeds, in the distance that came
+    with it or in its vector, a NaN among the neighbours, equal distances in the sub-graph
+    stage, and equal distances met only in the full-graph stage after more admissions than the
+    log holds (few candidates: H of them).  Vectors on a grid, so
+    that every distance is exact in any order of additions; rows, distances and statistics are
+    those of the array heaps, and two runs agree."""
+    from pilotann_b200 import extension
+    B, n, d, d_p = 12, 3000, 48, 16
+    g = torch.Generator().manual_seed(ef + n_cand)
+    p = make_problem(n=n, d=d, ratio=0.5, batch=B, n_init=32, seed=700)
+    full, q = (torch.round(p[x] * 128) / 128 for x in ("full", "query"))
+    if spoil.endswith("twins"):
+        at = torch.randperm(n, generator=g)
+        if spoil == "unsampled twins":
+            at = at[~torch.isin(at, p["nodelist"])]
+        at = at[:at.numel() // 2 * 2].view(2, -1)
+        full[at[0]] = full[at[1]]
+    ids = torch.stack([p["nodelist"][torch.randperm(p["nodelist"].numel(), generator=g)[:n_cand]]
+                       for _ in range(B)])
+    dist = ((q[:, :d_p].unsqueeze(1) - full[ids][:, :, :d_p]) ** 2).sum(-1)
+    hit = torch.arange(B) % 3 == 0                  # (the others may stay clean)
+    if spoil == "seed distance":
+        dist[hit, 5] = dist[hit, n_cand // 2] = float("nan")
+    elif spoil == "seed vector":
+        full[ids[hit][:, [3, n_cand - 1]].reshape(-1), d_p:] = float("nan")
+    elif spoil == "neighbour":
+        best = ids[hit].gather(1, dist[hit].argmin(1, keepdim=True)).reshape(-1)
+        bad = p["full_indices"].view(n, -1)[best, :2].reshape(-1)
+        full[bad] = float("nan")
+        dist[torch.isin(ids, bad)] = float("nan")
+    dist = dist.contiguous()
+    H = extension.cpu_heap_size_for(ef)
+    csr = [[p[a].contiguous(), p[b]] for a, b in (("indptr", "indices"), ("full_indptr", "full_indices"))]
+    want = [_on_array_heaps(ids[b], dist[b], q[b].double(), full.double(), *csr, k, ef, H, d_p)
+            for b in range(B)]
+    if spoil.endswith("twins"):                     # the case is what it claims to be
+        early, late = ([any(a[1] == b[1] and a[0] >= 0 for a, b in zip(w[i], w[i][1:max(k, 26) + 1]))
+                        for w in want] for i in (0, 1))
+        if spoil == "twins":
+            assert any(early)
+        else:
+            assert any(y and not x and w[3] > H for w, x, y in zip(want, early, late))
+    nbr, row_of = extension.pack_graph(p["indptr"].cuda(), p["indices"].cuda(), p["mapping"].cuda(),
+                                       p["storage"].size(0), 32)
+    full_nbr = extension.pack_fullgraph(p["full_indptr"].cuda(), p["full_indices"].cuda(), 32)
+    pool = extension.VisitedPool(n, 16)
+    for stage, top in ((0, None), (1, k)):
+        runs = []
+        for _ in range(2):
+            st = torch.zeros(B, 4, dtype=torch.int32, device="cuda")
+            got = extension.refine(ids.cuda(), dist.cuda(), q.cuda(), full.cuda(), nbr, row_of,
+                                   full_nbr, pool, ef, d_p, k=top, stats=st)
+            torch.cuda.synchronize()
+            runs.append([got[0].cpu(), got[1].cpu(), st.cpu()])
+        for x, y in zip(*runs):
+            assert torch.equal(x.nan_to_num(-7), y.nan_to_num(-7)) if x.is_floating_point() else torch.equal(x, y)
+        w_I = torch.tensor([[v for v, _ in w[stage]] for w in want])
+        w_D = torch.tensor([[dv for _, dv in w[stage]] for w in want])
+        w_st = torch.tensor([w[2] for w in want], dtype=torch.int32)
+        got_I, got_D, st = runs[0]
+        wrong = (got_I != w_I).any(1).nonzero().flatten().tolist()
+        assert not wrong, (top, wrong)
+        assert torch.equal(got_D.nan_to_num(-7, 1e30, -1e30), w_D.nan_to_num(-7, 1e30, -1e30)), top
+        assert torch.equal(st[:, :2 + 2 * stage], w_st[:, :2 + 2 * stage]), top
+
+
 @pytest.mark.skipif("PA_REFINE_PROFILE=1" not in os.environ.get("PILOTANN_B200_DEFINES", ""),
                     reason="needs a library built with PILOTANN_B200_DEFINES=PA_REFINE_PROFILE=1")
 @pytest.mark.parametrize("ef", [48, 257])
