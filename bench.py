@@ -51,10 +51,10 @@ OPERATING_EF = {2: 128}
 # the queries in that launch (bytes / query), stamped with the state of the kernel
 # it was captured on; None until captured
 NCU_TRAFFIC_PER_QUERY = {2: {
-    "traverse": {"bytes_per_query": (1.489819e9 + 7.637e6) / 1024,
-                 "captured_at": "library version 102 (kernel unchanged in 103), 1024 queries, ef 128"},
-    "refine": {"bytes_per_query": (11.408724e9 + 0.135678e9) / 1024,
-               "captured_at": "library version 103, 1024 queries, ef 128"}}}
+    "traverse": {"bytes_per_query": (1.488646e9 + 8.802e6) / 1024,
+                 "captured_at": "library version 104, 1024 queries, ef 128"},
+    "refine": {"bytes_per_query": (11.427216e9 + 0.139088e9) / 1024,
+               "captured_at": "library version 104, 1024 queries, ef 128"}}}
 PASSES = 10       # event-timed passes per step; a step's time is their median
 FALLBACK_HBM_GBS = 6650.0
 
@@ -730,12 +730,8 @@ def main():
         return total
 
     e2e_s = e2e_time(lambda: stage.search_host(q_host, ef, out_I=h_top_I, out_D=h_top_D, k=k))
-    e2e_chunked_s = e2e_time(lambda: stage.search_host(q_host, ef, chunk=256, out_I=h_top_I,
-                                                       out_D=h_top_D, k=k))
     e2e_stage_s = e2e_time(lambda: stage.search_host(q_host, ef, out_I=h_I, out_D=h_D,
                                                      rotated=h_rot))
-    e2e_stage_chunked_s = e2e_time(lambda: stage.search_host(q_host, ef, chunk=256, out_I=h_I,
-                                                             out_D=h_D, rotated=h_rot))
     h2d = q_host.numel() * 4          # per rank; the line reports world x these
     d2h = h_top_I.numel() * 8 + h_top_D.numel() * 4
     d2h_stage = h_I.numel() * 8 + h_D.numel() * 4 + h_rot.numel() * 4
@@ -794,13 +790,11 @@ def main():
     ref_traffic = NCU_TRAFFIC_PER_QUERY.get(cfg, {}).get("refine") if ef == 128 else None
 
     # ---- max over ranks ----
-    times = torch.tensor([total_ms, e2e_s * 1e3, sum(stage_step_ms), e2e_chunked_s * 1e3,
-                          e2e_stage_s * 1e3, e2e_stage_chunked_s * 1e3],
+    times = torch.tensor([total_ms, e2e_s * 1e3, sum(stage_step_ms), e2e_stage_s * 1e3],
                          dtype=torch.float64, device=device)
     if world > 1:
         torch.distributed.all_reduce(times, op=torch.distributed.ReduceOp.MAX)
-    total_ms, e2e_ms, stage_total_ms, e2e_chunked_ms, e2e_stage_ms, e2e_stage_chunked_ms = \
-        times.tolist()
+    total_ms, e2e_ms, stage_total_ms, e2e_stage_ms = times.tolist()
     if rank != 0:
         torch.distributed.destroy_process_group()
         return 0
@@ -837,8 +831,7 @@ def main():
                 "refinement (sub-graph stage and full-graph stage), top-k out",
         "recall": round(recall, 4), "ef_sweep": ef_sweep,
         "e2e": {"value": qps(e2e_ms), "unit": "queries/s", "h2d_bytes_per_step": world * h2d,
-                "d2h_bytes_per_step": world * d2h, "chunk": 0,
-                "chunk_256": {"value": qps(e2e_chunked_ms)}},
+                "d2h_bytes_per_step": world * d2h, "chunk": 0},
         "gpu_launches": launches, "passes_per_step": PASSES,
         "step_ms": {"min": min(step_ms), "median": statistics.median(step_ms),
                     "max": max(step_ms)},
@@ -851,8 +844,7 @@ def main():
         "stage": {"value": qps(stage_total_ms), "unit": "queries/s",
                   "ms_per_step": stage_total_ms / steps,
                   "e2e": {"value": qps(e2e_stage_ms), "h2d_bytes_per_step": world * h2d,
-                          "d2h_bytes_per_step": world * d2h_stage,
-                          "chunk_256": {"value": qps(e2e_stage_chunked_ms)}}},
+                          "d2h_bytes_per_step": world * d2h_stage}},
     }
     if world == 1 and not args.no_cpu:
         traverse_call()
