@@ -1482,7 +1482,9 @@ static int refine_launch_with(const RefineArgs &A, unsigned grid, int threads, i
 // have room a query gets the warps to fetch an expansion in one trip: 16 warps up to two
 // queries per SM, 8 up to four.  One query of 768 dimensions at ef 128: 0.86 -> 0.54 ms;
 // seven of 96 dimensions at ef 96: 0.32 -> 0.28; 333 of 384 dimensions at ef 48 (8 warps):
-// 0.47 -> 0.385.
+// 0.47 -> 0.385.  At the limits, ef 32 to 256, time over that of three or five warps: 16 warps
+// at two queries per SM 0.65 to 0.84 (96 dimensions up to 0.97, where 8 are as fast), 8 warps at four
+// 0.83 to 0.96, sub-graph stage alone included.
 template <int R>
 static int refine_launch_for(const RefineArgs &A, unsigned grid, unsigned sms, int dev,
                              cudaStream_t stream) {

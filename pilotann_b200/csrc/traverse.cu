@@ -468,56 +468,56 @@ __device__ __forceinline__ float list_at(const float (&cd)[4], unsigned p) {
 // + n_teams, ... below j_end.  The loop bound is the same for every lane of
 // a warp (the team shuffles name the whole warp); lanes past the end carry
 // a false predicate.  `spare`: 32 slots behind the candidates, one per lane.
-        template <class Layout>
+template <class Layout>
 __device__ __forceinline__ void team_distances(const Layout &L, int2 *slots, float *cand_d,
                                                int spare, const float *q_s, int d, int lane,
                                                int team, int n_teams, int j_begin, int j_end) {
-            const int t8 = lane & 7;
-            for (int jb = j_begin; jb < j_end; jb += 2 * n_teams) {
-                const int j0 = jb + team;
-                const int j1 = j0 + n_teams;
-                const bool p0_in = j0 < j_end, p1_in = j1 < j_end;
-                // Lanes past the end or without a vector read row 0 and drop the
-                // result: every load below is unconditional, no lane-dependent branch.
-                // (j0, j1 stay inside the arrays: they are below j_end + 2 * n_teams.)
-                int2 s0 = slots[j0], s1 = slots[j1];
-                if constexpr (!Layout::kPacked) {
-                    s0.y = static_cast<int32_t>(__ldg(L.mapping + (p0_in ? s0.x : 0)));
-                    s1.y = static_cast<int32_t>(__ldg(L.mapping + (p1_in ? s1.x : 0)));
-                    slots[(t8 == 0 && p0_in) ? j0 : spare + lane].y = s0.y;
-                    slots[(t8 == 0 && p1_in) ? j1 : spare + lane].y = s1.y;
-                }
-                const bool p0 = p0_in && s0.y >= 0, p1 = p1_in && s1.y >= 0;
-                const float *r0 = L.storage + static_cast<int64_t>(p0 ? s0.y : 0) * d;
-                const float *r1 = L.storage + static_cast<int64_t>(p1 ? s1.y : 0) * d;
-                float a0 = 0.0f, a1 = 0.0f;
-                for (int o = 4 * t8; o < d; o += 128) {
-                    // up to four stripes of each row in flight before any arithmetic
-                    float4 x0[4], x1[4];
+    const int t8 = lane & 7;
+    for (int jb = j_begin; jb < j_end; jb += 2 * n_teams) {
+        const int j0 = jb + team;
+        const int j1 = j0 + n_teams;
+        const bool p0_in = j0 < j_end, p1_in = j1 < j_end;
+        // Lanes past the end or without a vector read row 0 and drop the
+        // result: every load below is unconditional, no lane-dependent branch.
+        // (j0, j1 stay inside the arrays: they are below j_end + 2 * n_teams.)
+        int2 s0 = slots[j0], s1 = slots[j1];
+        if constexpr (!Layout::kPacked) {
+            s0.y = static_cast<int32_t>(__ldg(L.mapping + (p0_in ? s0.x : 0)));
+            s1.y = static_cast<int32_t>(__ldg(L.mapping + (p1_in ? s1.x : 0)));
+            slots[(t8 == 0 && p0_in) ? j0 : spare + lane].y = s0.y;
+            slots[(t8 == 0 && p1_in) ? j1 : spare + lane].y = s1.y;
+        }
+        const bool p0 = p0_in && s0.y >= 0, p1 = p1_in && s1.y >= 0;
+        const float *r0 = L.storage + static_cast<int64_t>(p0 ? s0.y : 0) * d;
+        const float *r1 = L.storage + static_cast<int64_t>(p1 ? s1.y : 0) * d;
+        float a0 = 0.0f, a1 = 0.0f;
+        for (int o = 4 * t8; o < d; o += 128) {
+            // up to four stripes of each row in flight before any arithmetic
+            float4 x0[4], x1[4];
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const bool in = o + 32 * m < d;
-                        x0[m] = in ? __ldg(reinterpret_cast<const float4 *>(r0 + o + 32 * m))
-                                   : make_float4(0, 0, 0, 0);
-                        x1[m] = in ? __ldg(reinterpret_cast<const float4 *>(r1 + o + 32 * m))
-                                   : make_float4(0, 0, 0, 0);
-                    }
+            for (int m = 0; m < 4; ++m) {
+                const bool in = o + 32 * m < d;
+                x0[m] = in ? __ldg(reinterpret_cast<const float4 *>(r0 + o + 32 * m))
+                           : make_float4(0, 0, 0, 0);
+                x1[m] = in ? __ldg(reinterpret_cast<const float4 *>(r1 + o + 32 * m))
+                           : make_float4(0, 0, 0, 0);
+            }
 #pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        if (o + 32 * m < d) {
-                            const float4 qa = *reinterpret_cast<const float4 *>(q_s + o + 32 * m);
-                            a0 = stripe(a0, qa, x0[m]);
-                            a1 = stripe(a1, qa, x1[m]);
-                        }
-                    }
+            for (int m = 0; m < 4; ++m) {
+                if (o + 32 * m < d) {
+                    const float4 qa = *reinterpret_cast<const float4 *>(q_s + o + 32 * m);
+                    a0 = stripe(a0, qa, x0[m]);
+                    a1 = stripe(a1, qa, x1[m]);
                 }
-                a0 = team_reduce(a0);
-                a1 = team_reduce(a1);
-                // +inf marks a candidate without a vector: it is never inserted
-                cand_d[(t8 == 0 && p0_in) ? j0 : spare + lane] = p0 ? a0 : CUDART_INF_F;
-                cand_d[(t8 == 0 && p1_in) ? j1 : spare + lane] = p1 ? a1 : CUDART_INF_F;
             }
         }
+        a0 = team_reduce(a0);
+        a1 = team_reduce(a1);
+        // +inf marks a candidate without a vector: it is never inserted
+        cand_d[(t8 == 0 && p0_in) ? j0 : spare + lane] = p0 ? a0 : CUDART_INF_F;
+        cand_d[(t8 == 0 && p1_in) ? j1 : spare + lane] = p1 ? a1 : CUDART_INF_F;
+    }
+}
 
 template <int H, int CH, class Layout>
 __global__ void __launch_bounds__(kThreads, PA_MIN_CTAS)
@@ -1018,12 +1018,14 @@ traverse_kernel(Layout L, int64_t *__restrict__ out_I, float *__restrict__ out_D
 // candidate), so its neighbour row is on its way while they run.
 //
 // It takes three times the heap instructions of the kernel above, which keeps four
-// heaps in step in one warp, so it pays while an SM has one or two queries.  Search
-// without refinement, four warps / eight warps, us: 1 million vectors, 128 dimensions at
-// ef 128: 1 query 598 / 518, 148 835 / 641, 296 867 / 737, 444 899 / 882, 592 923 / 1005; 96
-// dimensions at ef 48: 148 263 / 236, 296 275 / 266, 444 298 / 329; 64 dimensions at ef 128
-// in clusters: 148 185 / 164, 296 197 / 208, 444 240 / 265.  Sixteen warps: 543, 623, 754 at
-// the first three sizes.
+// heaps in step in one warp, so it pays while an SM has one or two queries.  Time with eight
+// warps over time with four, ef 24 to 256 (three million-vector collections and one of 100 k,
+// their reduced dimensions, 32 and 192; rows in the L2 and flushed alike): up to one query per SM
+// 0.66 to 0.91, one and a half 0.73 to 0.98, two 0.74 to 0.97, three 0.82 to 1.15, four 0.89 to
+// 1.34, five 1.05 to 1.59.  At three it is the rows that decide, 192 dimensions 0.82 to 0.98, fewer
+// up to 1.15.  E.g. 64 dimensions in clusters at ef 128: two per SM 0.90, three 0.91,
+// four 1.01; 128 dimensions 0.85, 0.98, 1.12.  (Sixteen warps were better only for a single
+// query per SM and 64 rounds and more.)
 constexpr int kWideThreads = 256;
 constexpr int kWidePerSm = 2;  // up to this many queries per SM
 
